@@ -20,6 +20,10 @@ namespace kda {
 
 constexpr int PLAN_THREADS = 1024;
 constexpr int SORT_MAX = 4096;
+// Up to this many sequences the tables are compared pairwise at once, beyond it a pass over the table looks first whether
+// that is needed.  This kernel back to back on a B200, pairwise / with the passes: ascending checkpoint rows 3 sequences
+// 6.15 / 6.41 us, 5 sequences 6.39 / 6.61, 6 sequences 7.18 / 6.66; one sequence with a slot table 5.8 / 6.15.
+constexpr int PAIRWISE_MAX = 5;
 constexpr int RANK_MAX = 512;            // sequences ordered by counting; beyond, the sorting network has fewer steps
 // cut planning
 constexpr int CUT_MAX_SEQS = 1024;       // sequences a cut plan is made for (beyond: never cut)
@@ -59,7 +63,7 @@ __global__ void __launch_bounds__(PLAN_THREADS, 1) kda_plan_kernel(const PlanPar
   // the chunk kernel chained behind this launch may become resident now (it waits for this kernel's results itself)
   asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
   if (tid == 0) { s_bits = 0; s_overlap = 0; s_slot_dup = 0; s_ck_order = 0; }
-  const bool hashed = a.dst_idx != nullptr && N <= SORT_MAX / 2;     // the sort keys' memory serves as the hash set first
+  const bool hashed = a.dst_idx != nullptr && N > PAIRWISE_MAX && N <= SORT_MAX / 2;     // the sort keys' memory serves as the hash set first
   if (hashed)
     for (int i = tid; i < SORT_MAX; i += bd) keys[i] = ~0ULL;
   __syncthreads();
@@ -91,26 +95,30 @@ __global__ void __launch_bounds__(PLAN_THREADS, 1) kda_plan_kernel(const PlanPar
   // ---- fast checks: are the destination slots all different (hash set), do the checkpoint rows of every sequence lie
   // behind those of the one before?
   const bool cks = a.ck_base != nullptr && a.ck_every > 0;
-  for (int i = tid; i < N; i += bd) {
-    if (a.dst_idx != nullptr) {
-      const long long d = rd_table(a.dst_idx, a.dst_is64, i);
-      if (!hashed) s_slot_dup = 1;
-      else if (d >= 0 && d < a.dst_slots) {
-        for (unsigned at = (unsigned)d * 2654435761u >> 20;; at++) {            // 4096 entries, at most half of them used
-          const unsigned long long old = atomicCAS(&keys[at & (SORT_MAX - 1)], ~0ULL, (unsigned long long)d);
-          if (old == ~0ULL) break;
-          if (old == (unsigned long long)d) { s_slot_dup = 1; break; }
+  bool slot_dup = !hashed, ck_search = true;
+  if (N > PAIRWISE_MAX) {
+    for (int i = tid; i < N; i += bd) {
+      if (a.dst_idx != nullptr) {
+        const long long d = rd_table(a.dst_idx, a.dst_is64, i);
+        if (!hashed) s_slot_dup = 1;
+        else if (d >= 0 && d < a.dst_slots) {
+          for (unsigned at = (unsigned)d * 2654435761u >> 20;; at++) {          // 4096 entries, at most half of them used
+            const unsigned long long old = atomicCAS(&keys[at & (SORT_MAX - 1)], ~0ULL, (unsigned long long)d);
+            if (old == ~0ULL) break;
+            if (old == (unsigned long long)d) { s_slot_dup = 1; break; }
+          }
         }
       }
+      if (cks && i > 0) {
+        long long v, cnt, vp, cp;
+        const bool ok = ck_range(i, v, cnt), okp = ck_range(i - 1, vp, cp);
+        if (!ok || !okp || v < vp + cp) s_ck_order = 1;
+      }
     }
-    if (cks && i > 0) {
-      long long v, cnt, vp, cp;
-      const bool ok = ck_range(i, v, cnt), okp = ck_range(i - 1, vp, cp);
-      if (!ok || !okp || v < vp + cp) s_ck_order = 1;
-    }
+    __syncthreads();
+    slot_dup = s_slot_dup != 0;
+    ck_search = s_ck_order != 0;
   }
-  __syncthreads();
-  const bool slot_dup = s_slot_dup != 0, ck_search = s_ck_order != 0;
 
   // ---- per-sequence tables
   for (int i = tid; i < N; i += bd) {
@@ -200,7 +208,7 @@ __global__ void __launch_bounds__(PLAN_THREADS, 1) kda_plan_kernel(const PlanPar
 
   // ---- order: longest first, ties by index (bitonic sort of (len descending, index) keys)
   const bool sorted = N <= SORT_MAX;
-  if (N <= RANK_MAX) {
+  if (N > 1 && N <= RANK_MAX) {         // (one sequence: the network has no stage)
     // position = number of smaller keys (they are all different); bd / n2 threads share the comparisons of a key
     int n2 = 1;
     while (n2 < N) n2 <<= 1;
