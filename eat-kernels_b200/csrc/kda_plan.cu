@@ -24,7 +24,13 @@ constexpr int SORT_MAX = 4096;
 // that is needed.  This kernel back to back on a B200, pairwise / with the passes: ascending checkpoint rows 3 sequences
 // 6.15 / 6.41 us, 5 sequences 6.39 / 6.61, 6 sequences 7.18 / 6.66; one sequence with a slot table 5.8 / 6.15.
 constexpr int PAIRWISE_MAX = 5;
-constexpr int RANK_MAX = 512;            // sequences ordered by counting; beyond, the sorting network has fewer steps
+// Up to this many sequences the order is found by counting: every key against every other, about N * n2 / 1024 steps of a
+// thread (n2: N rounded up to a power of two), beyond it by a sorting network of log2(n2) (log2(n2) + 1) / 2 stages with a
+// barrier each.  This kernel back to back on a B200, counting / network: 48 sequences 6.15 / 8.2 us, 256 8.2 / 10.6, 320
+// 12.3 / 12.8, 384 13.4 / 13.9, 416 14.34 / 14.34 (with checkpoint rows 15.5 / 14.4), 480 15.5 / 14.3, 512 16.4 / 14.3,
+// 513 24.6 / 18.4, 1024 44.4 / 20.5.
+constexpr int RANK_MAX = 384;
+constexpr int RANK_SLOTS = 512;          // RANK_MAX rounded up to a power of two
 // cut planning
 constexpr int CUT_MAX_SEQS = 1024;       // sequences a cut plan is made for (beyond: never cut)
 constexpr int N_CAND = 9;                // candidate piece lengths
@@ -55,7 +61,7 @@ __global__ void __launch_bounds__(PLAN_THREADS, 1) kda_plan_kernel(const PlanPar
   __shared__ unsigned long long keys[SORT_MAX];
   __shared__ unsigned char s_keep[SORT_MAX];     // checkpoint rows of sequence i: 0 = none / rejected, 1 = kept
   __shared__ int s_bits, s_overlap, s_slot_dup, s_ck_order;
-  __shared__ int s_rank[RANK_MAX];
+  __shared__ int s_rank[RANK_SLOTS];
   __shared__ int s_lp, s_cmax, s_uncut_work, s_work[N_CAND], s_pieces[N_CAND], s_longest[N_CAND], s_ncut[N_CAND];
   __shared__ unsigned short s_off_a[CUT_MAX_SEQS], s_off_b[CUT_MAX_SEQS];
   __shared__ unsigned char s_cnt_a[CUT_MAX_SEQS], s_cnt_b[CUT_MAX_SEQS], s_off_m[CUT_MAX_SEQS], s_off_c[CUT_MAX_SEQS];

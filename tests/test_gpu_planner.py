@@ -71,7 +71,7 @@ def _short_lengths(N, rng):
 
 
 @pytest.mark.parametrize("repeat", [False, True])
-@pytest.mark.parametrize("N", [1, 2, 5, 6])
+@pytest.mark.parametrize("N", [1, 2, 5, 6, 384, 385, 512, 513])
 def test_slots_and_order(N, repeat):
     rng = random.Random(N)
     lens = _short_lengths(N, rng)
