@@ -71,7 +71,7 @@ def _short_lengths(N, rng):
 
 
 @pytest.mark.parametrize("repeat", [False, True])
-@pytest.mark.parametrize("N", [1, 2, 5, 6, 384, 385, 512, 513])
+@pytest.mark.parametrize("N", [1, 2, 5, 6, 384, 385, 512, 513, 1025, 2048, 2049, 4096, 4097])
 def test_slots_and_order(N, repeat):
     rng = random.Random(N)
     lens = _short_lengths(N, rng)
@@ -83,7 +83,35 @@ def test_slots_and_order(N, repeat):
 
 @pytest.mark.parametrize("lens,starts,kept", [
     ([100], [1], [0]), ([100, 33], [2, 0], [0, 1]), ([100, 33], [0, 3], [0]),
-    ([100, 33, 0, 1, 64], [5, 3, 0, 2, 0], [0, 1, 2, 3, 4]), ([100, 33, 0, 1, 64], [0, 4, 0, 6, 5], [0, 1, 2, 3])])
+    ([100, 33, 0, 1, 64], [5, 3, 0, 2, 0], [0, 1, 2, 3, 4]), ([100, 33, 0, 1, 64], [0, 4, 0, 6, 5], [0, 1, 2, 3]),
+    ([100, 33, 1, 64, 31, 32, 1], [0, 4, 6, 7, 9, 10, 11], [0, 1, 2, 3, 4, 5, 6]),         # ascending
+    ([100, 33, 1, 64, 31, 32, 1], [8, 6, 5, 3, 2, 1, 0], [0, 1, 2, 3, 4, 5, 6]),           # descending
+    ([100, 33, 0, 64, 0, 32, 0, 0], [0, 4, 6, 6, 0, 8, 0, 0], list(range(8))),             # empty sequences padded with 0
+    ([100, 33, 1, 64, 31, 32, 1], [0, 4, 6, 7, 9, 10, 2], [0, 1, 2, 3, 4, 5]),             # the last one into the first's rows
+    ([100, 33, 64, 64, 31, 32, 1], [0, 3, 4, 6, 8, 9, 10], [0, 2, 3, 4, 5, 6])])           # a rejected one blocks nobody
 def test_checkpoint_tables(lens, starts, kept):
     """Checkpoint rows every 32 tokens: ranges that go down, holes, empty sequences at row 0, overlaps."""
-    assert _serving_call(lens, random.Random(2).sample(range(9), len(lens)), 9, 60 + len(lens), 32, starts, 10)[1] == kept
+    assert _serving_call(lens, random.Random(2).sample(range(9), len(lens)), 9, 60 + len(lens), 32, starts, 12)[1] == kept
+
+
+def test_slots_with_one_hash_entry():
+    """Slots whose first entry in the planner's hash set (4096 entries, Fibonacci hashing) is one of four neighbours
+    around the end of the set: they probe one another's entries and wrap; one of them is repeated behind them all."""
+    P = 16384
+    slots = [d for d in range(P) if (d * 2654435761 % 2**32 >> 20) in (4094, 4095, 0, 1)]
+    assert len(slots) > 8
+    random.Random(5).shuffle(slots)
+    lens = _short_lengths(len(slots), random.Random(6))
+    _serving_call(lens, slots, P, 70)
+    _serving_call(lens + [3], slots + [slots[1]], P, 71)
+
+
+@pytest.mark.parametrize("N", [384, 385, 1024, 1025])
+def test_cuts_follow_either_order(N):
+    """One long sequence among many short ones is cut, whichever way the tasks were ordered (up to 1024 sequences)."""
+    rng = random.Random(N)
+    lens = [rng.randint(1, 8) for _ in range(N)]
+    lens[N // 2] = 4096
+    launch, _ = _serving_call(lens, rng.sample(range(N + 5), N), N + 5, 80)
+    na, nb, cut = launch.plan_counts()
+    assert cut == (1 if N <= 1024 else 0) and na + nb >= N, (na, nb, cut)
