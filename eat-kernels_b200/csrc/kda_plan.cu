@@ -42,7 +42,10 @@ constexpr int DUAL_X8 = 9;               // a dual-chain chunk step without outp
 __device__ __forceinline__ long long map_task_cost(int lp, int dual) {
   return dual ? (long long)(DUAL_X8 * lp + 7) / 8 + TASK_OVERHEAD : 2LL * (lp + TASK_OVERHEAD);
 }
-constexpr int SCAN_STEPS_X16 = 12;       // one map of the scan chain, in 1/16 chunk steps
+// One map of the scan chain, in 1/16 chunk steps.  An underestimate: a map takes 5.1 us value-first and 6.1 us key-first on
+// up to 16 heads (slope from 1 to 14 maps of one chain), about two chunk steps, so the model undercharges a cut by more
+// than one chunk step per map.
+constexpr int SCAN_STEPS_X16 = 12;
 constexpr int LAUNCH_STEPS = 4;          // the scan launch and the second kernel launch, in chunk steps
 __host__ __device__ constexpr int cand_pieces(int k) { return k < 3 ? k + 2 : (k == 3 ? 6 : (k == 4 ? 8 : (k == 5 ? 12 : (k == 6 ? 16 : (k == 7 ? 24 : 32))))); }
 
@@ -50,13 +53,16 @@ __device__ __forceinline__ long long rd_table(const void* p, int is64, long long
   return is64 ? reinterpret_cast<const long long*>(p)[i] : (long long)reinterpret_cast<const int*>(p)[i];
 }
 
-// One CTA of latency in front of every launch, so what counts is the longest chain of dependent steps: table checks that
-// hold for every well-formed table in a pass (a hash set of the slots, neighbouring checkpoint ranges) with the pairwise
-// loops behind them only for tables that fail it; a rank by counting instead of a sorting network up to RANK_MAX
-// sequences; one lane per candidate of the cut model (its divisions are 64 bits wide), one thread per piece of a cut
-// sequence.  Measured on a B200 over whole calls, before -> after: 48 sequences with checkpoint rows and cuts (8 heads)
-// 394.7 -> 364.0 us, 512 sequence slots 1339 -> 1318 us, one cut sequence of 32 768 tokens 1026 -> 1014 us, 7 short
-// sequences 140.9 -> 137.9 us.
+// One CTA of latency in front of every launch, so what counts is the longest chain of dependent steps.
+//   Checks: one pass tells whether the slots are all different (a hash set) and whether each sequence's checkpoint rows lie
+//   behind those of the sequence before it; the pairwise loops, which resolve repeats and overlaps, follow only if not.
+//   Valid tables that take them all the same: more than SORT_MAX / 2 slots (the hash set would be more than half full) and
+//   checkpoint rows that do not ascend with the sequences, rows 0 given to empty sequences among them.
+//   Order: by counting or by a sorting network (RANK_MAX).  Cuts: one lane per candidate of the cost model (its divisions
+//   are 64 bits wide), one warp per cut sequence and one lane per piece of it when the pieces are written.
+// Back to back on a B200, without cuts: one sequence 5.1 us, 48 with slots 6.2 us and with ascending checkpoint rows 7.2 us
+// (10.3 and 20.5 us when every check is pairwise), 512 with slots 14.4 us (38.9 us), 2048 36.9 us (197 us); pairwise loops
+// that have to run: 512 sequences with descending checkpoint rows 88 us, 2049 slots 226 us.
 __global__ void __launch_bounds__(PLAN_THREADS, 1) kda_plan_kernel(const PlanParams a) {
   __shared__ unsigned long long keys[SORT_MAX];
   __shared__ unsigned char s_keep[SORT_MAX];     // checkpoint rows of sequence i: 0 = none / rejected, 1 = kept
@@ -98,8 +104,8 @@ __global__ void __launch_bounds__(PLAN_THREADS, 1) kda_plan_kernel(const PlanPar
   }
   __syncthreads();
 
-  // ---- fast checks: are the destination slots all different (hash set), do the checkpoint rows of every sequence lie
-  // behind those of the one before?
+  // ---- do the tables need the pairwise loops: are the destination slots all different (hash set), do the checkpoint rows
+  // of every sequence lie behind those of the one before?
   const bool cks = a.ck_base != nullptr && a.ck_every > 0;
   bool slot_dup = !hashed, ck_search = true;
   if (N > PAIRWISE_MAX) {
@@ -212,7 +218,7 @@ __global__ void __launch_bounds__(PLAN_THREADS, 1) kda_plan_kernel(const PlanPar
     __syncthreads();
   }
 
-  // ---- order: longest first, ties by index (bitonic sort of (len descending, index) keys)
+  // ---- order: longest first, ties by index ((len descending, index) keys; counting up to RANK_MAX, then a bitonic network)
   const bool sorted = N <= SORT_MAX;
   if (N > 1 && N <= RANK_MAX) {         // (one sequence: the network has no stage)
     // position = number of smaller keys (they are all different); bd / n2 threads share the comparisons of a key
