@@ -118,8 +118,7 @@ void fill_chunk_params(kda::ChunkParams& p, const KdaPrefillArgs* a) {
   p.prof = g_prof;
 }
 
-// Tensor maps of the token tensors for the tcgen05 kernel's copy engine (q, k, v in 64-channel halves with the 128-byte
-// swizzle, g as whole 128-channel rows).  T == 0: nothing is ever copied, the maps stay zeroed.
+// Tensor maps of the token tensors for the tcgen05 kernel's copy engine (see kda_tma.cuh).  T == 0: nothing is ever copied, the maps stay zeroed.
 // A prepared launch calls with the same pointers and strides every time, so the encoded maps are kept per thread
 // (a few entries, replaced round-robin) instead of going through the driver's encoder at every launch.
 struct MapKey {
@@ -147,10 +146,10 @@ int fill_tma_maps(kda::TmaMaps& m, const KdaPrefillArgs* a) {
       return KDA_OK;
     }
   const bool plain = a->frontend == KDA_FRONTEND_PLAIN;
-  int rc = kda::encode_token_map(&m.q, a->q, 2, false, a->T, a->H, a->ldq, 64, true);
-  if (rc == 0) rc = kda::encode_token_map(&m.k, a->k, 2, false, a->T, a->H, a->ldk, 64, true);
-  if (rc == 0) rc = kda::encode_token_map(&m.v, a->v, 2, false, a->T, a->H, a->ldv, 64, true);
-  if (rc == 0) rc = kda::encode_token_map(&m.g, a->g, plain ? 4 : 2, plain, a->T, a->H, a->ldg, 128, false);
+  int rc = kda::encode_token_map(&m.q, a->q, false, a->T, a->H, a->ldq);
+  if (rc == 0) rc = kda::encode_token_map(&m.k, a->k, false, a->T, a->H, a->ldk);
+  if (rc == 0) rc = kda::encode_token_map(&m.v, a->v, false, a->T, a->H, a->ldv);
+  if (rc == 0) rc = kda::encode_token_map(&m.g, a->g, plain, a->T, a->H, a->ldg);
   if (rc != 0) {
     snprintf(g_cuda_err, sizeof(g_cuda_err), "cuTensorMapEncodeTiled failed (%d)", rc);
     return KDA_ERR_LAUNCH;

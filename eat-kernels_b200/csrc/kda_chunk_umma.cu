@@ -31,6 +31,14 @@
 // the two results pulled out of tensor memory by the inverse warps.  It halves the work of the preparation warps, but
 // the tensor-core round trip (issue, commit, barrier, tensor-memory load) and the extraction sit on the chain
 // tiles -> products -> inverse -> MMA2, which with two operand stages is what sets the per-chunk time: 3-13 % slower.
+//
+// What bounds it: with 28 warps every warp issues about one instruction per ten cycles, so a chunk lasts as long as the chain
+// [kd ; qd] free -> operand tiles -> intra-chunk products -> inverse -> MMA2 over the two stages; the tensor pipe needs 970
+// cycles of it (the MMAs of a chunk depend on one another and still issue back to back).  Cumulative decay in the lanes of one
+// warp, norms off that chain, an inverse that no longer waits for v and a third q / k stage for raw gates, whole calls on a
+// B200 before / after: 8 x 1024 tokens at 64 heads, raw 419 / 394 us; 1 x 8192 at 96 heads, raw 788 / 721; 1 x 32768 at 16
+// heads with checkpoints, raw 1022 / 953; 16 x U[128, 4096] at 32 heads, plain 573 / 553; 48 requests at 64 heads, plain
+// 1803 / 1711.
 #include "kda_common.cuh"
 #include "kda_plan.cuh"
 #include "kda_tma.cuh"
@@ -47,30 +55,40 @@ constexpr int W_MMA = 0, W_INV0 = 1, W_LOAD = 3, W_SCALE0 = 4, W_PREP0 = 12;
 constexpr int PREP_GROUPS = 2;                 // group g prepares the chunks c with c % 2 == g, in stage g
 constexpr int PREP_WARPS = 8, PREP_THREADS = 256;   // per group
 
-// ---- shared memory map (bytes); operand tiles are 1024-byte aligned
-constexpr int CS_KDQD = 0, CS_KR = 32768, CS_V = 49152, CS_TB = 57344, CS_M = 61440, CS_STAGE = 65536;
-constexpr int OFF_CONS = 0;                                   // 2 stages
-constexpr int RAW_G = 0, RAW_Q = 16384, RAW_K = 24576, RAW_STAGE = 32768;
-constexpr int OFF_RAW = OFF_CONS + 2 * CS_STAGE;              // 2 stages
-constexpr int OFF_KIS = OFF_RAW + 2 * RAW_STAGE;              // 2 x 8192 (one per prep group)
-constexpr int OFF_TBH = OFF_KIS + 2 * 8192;                   // 2 x 2048 (bf16, 64-byte swizzle)
-constexpr int OFF_L = OFF_TBH + 4096;                         // 2 x 4096 fp32 [32][32]
-constexpr int OFF_DEC = OFF_L + 8192;                         // 4 x 512 (a slot is rewritten four chunks later)
-constexpr int OFF_FR = OFF_DEC + 2048;                        // per prep group: (free), 2^r, first-half sum then 2^(G31-r) : 2 x 3 x 512
-constexpr int OFF_BETA = OFF_FR + 2 * 1536;                   // raw-stage beta: 2 x 128
-constexpr int OFF_LBETA = OFF_BETA + 256;                     // beta next to L: 2 x 128
+// ---- shared memory map (bytes); operand tiles are 1024-byte aligned.  A stage holds the operands of one chunk: what the
+// tensor core reads (CS_*) and the bf16 k tile of the intra-chunk products (KI).
+constexpr int CS_KDQD = 0, CS_KR = 32768, CS_V = 49152, CS_TB = 57344, CS_M = 61440;
+constexpr int KI = 65536, STAGE = KI + 8192;
+// Raw tiles: a ring of gate tiles and a ring of q / k tiles in 64 KB (the decayed bf16 tiles of the intra-chunk products
+// replace q and k in place).  bf16 gates (8 KB) leave room for a third q / k stage.
+template <int FE> struct Raw {
+  static constexpr int G_BYTES = FE == 1 ? 16384 : 8192, NQK = FE == 1 ? 2 : 3;
+  // The full barriers belong to chunks c, c + NFULL, ..: always the same preparation group waits on one, so it sees every
+  // phase of it (a group that skipped a phase could take an older one of the same parity for its own).
+  static constexpr int NFULL = NQK == 3 ? 6 : 2;
+  static constexpr int OFF_G = 2 * STAGE, OFF_QK = OFF_G + 2 * G_BYTES;      // q, then k, of a stage
+  static_assert(2 * G_BYTES + NQK * 16384 == 65536, "raw tiles");
+};
+constexpr int OFF_NORM = 2 * STAGE + 65536;                   // raw gates: partial square sums, 2 x [channel half]{q, k}[token]
+constexpr int OFF_TBH = OFF_NORM + 1024;                      // 2 x 2048 (bf16, 64-byte swizzle)
+constexpr int LS = 40;                                        // row stride of L in floats: rows 8 banks apart, 16-byte aligned
+constexpr int OFF_L = OFF_TBH + 4096;                         // 2 x fp32 [32][LS]
+constexpr int OFF_DEC = OFF_L + 2 * C * LS * 4;               // 4 x 512 (a slot is rewritten four chunks later)
+constexpr int OFF_BETA = OFF_DEC + 2048;                      // beta of a chunk: 2 groups x 2 (alternating) x 128
+constexpr int OFF_LBETA = OFF_BETA + 512;                     // beta next to L: 2 x 128
 constexpr int OFF_BAR = OFF_LBETA + 256;                      // mbarriers
-constexpr int NUM_BARS = 42;
+constexpr int NUM_BARS = 43;
 constexpr int OFF_MISC = OFF_BAR + NUM_BARS * 8;              // +0 tmem slot, +8 abort code, +12 range flag, +16 wait limit (ns)
 constexpr int SMEM_BYTES = OFF_MISC + 64;
-static_assert(SMEM_BYTES <= 227 * 1024, "shared memory budget");
+static_assert(SMEM_BYTES <= 227 * 1024 && STAGE % 1024 == 0 && OFF_MISC % 8 == 0, "shared memory budget");
 
 // mbarrier indices
 constexpr int B_G_FULL = 0, B_G_EMPTY = 2, B_CONS_EMPTY = 4, B_P1_FULL = 6, B_INV_FULL = 8, B_L_FULL = 10,
               B_L_EMPTY = 12, B_O_FULL = 14, B_O_EMPTY = 16, B_MMA1_DONE = 18, B_S_READY = 19, B_DRAIN = 20, B_V_EMPTY = 21,
-              B_QK_FULL = 23, B_QK_EMPTY = 25, B_V_FULL = 27, B_KDQD_EMPTY = 29,
-              B_MMA1_DONE_T = 31, B_S_READY_T = 32,   // second chain of a dual-chain task
-              B_TOT = 34;                             // 2 groups x 4 warp pairs: first-half sums of step A
+              B_QK_FULL = 23, B_QK_EMPTY = 29, B_V_FULL = 32, B_KDQD_EMPTY = 34,
+              B_MMA1_DONE_T = 36, B_S_READY_T = 37,   // second chain of a dual-chain task
+              B_NORM = 38,                            // partial square sums of q and k (raw gates only)
+              B_KDQD_FULL = 40;                       // [kd ; qd] written: MMA1 may start before the rest of the stage is
 
 // tensor-memory columns
 constexpr uint32_t TM_COLS = 512, TM_S = 0, TM_WO = 128, TM_U = 256;
@@ -136,13 +154,14 @@ __device__ __noinline__ bool loader_idle_expired(unsigned long long idle_ns, vol
 // Before the CTA may leave, every copy the loader issued has landed (on the normal path the consumers saw to that
 // long ago and these waits return at once; after a give-up they keep the copy engine from writing into a dead CTA).
 // A stage's full barrier is not re-armed after its last copy, so the parity of that last phase is still testable.
-__device__ __noinline__ void loader_drain(uint32_t bars, volatile int* abort_flag, int cg, int cq, int cv) {
+__device__ __noinline__ void loader_drain(uint32_t bars, volatile int* abort_flag, int cg, int cq, int cv, int nfull) {
 #pragma unroll 1
   for (int st = 0; st < 3; st++) {
     const int issued = st == 0 ? cg : (st == 1 ? cq : cv);
     const int fb = st == 0 ? B_G_FULL : (st == 1 ? B_QK_FULL : B_V_FULL);
-    for (int c = max(0, issued - 2); c < issued; c++)
-      if (!mbar_wait_drain(bars + 8u * (uint32_t)(fb + (c & 1)), (uint32_t)((c >> 1) & 1), abort_flag))
+    const int nb = st == 1 ? nfull : 2;
+    for (int c = max(0, issued - nb); c < issued; c++)
+      if (!mbar_wait_drain(bars + 8u * (uint32_t)(fb + c % nb), (uint32_t)((c / nb) & 1), abort_flag))
         atomicCAS(const_cast<int*>(abort_flag), 0, E_DRAIN + fb);
   }
 }
@@ -156,34 +175,35 @@ __device__ void role_loader(const ChunkParams& p, const TmaMaps& m, const Ctx& x
   // suspend time, and the refill latency of q / k sits on the chain  copy -> step B -> step C -> inverse -> MMA2.
   if (lane != 0) return;
   const int n = x.nchunks;
+  typedef Raw<FE> R;
   int cg = 0, cq = 0, cv = 0;                 // next chunk of each stream
+  int sq = 0;                                 // q / k stage of chunk cq, and the parity of its empty barrier
+  uint32_t pq = 1;
   unsigned idle = 0;
   unsigned long long t_idle = 0;
 #pragma unroll 1
   while (cg < n || cq < n || cv < n) {
     bool progressed = false;
     if (cq < n) {
-      const int s = cq & 1;
-      if (mbar_test_wait(x.bar(B_QK_EMPTY + s), (uint32_t)(((cq >> 1) & 1) ^ 1))) {
-        uint8_t* raw = x.smem + OFF_RAW + s * RAW_STAGE;
-        const uint32_t qraw = smem_u32(raw + RAW_Q), kraw = smem_u32(raw + RAW_K);
+      if (mbar_test_wait(x.bar(B_QK_EMPTY + sq), pq)) {
+        const uint32_t raw = smem_u32(x.smem + R::OFF_QK + sq * 16384);
         const int tok0 = (int)(x.t0 + (long long)cq * C);
-        tma::mbar_arrive_expect_tx(x.bar(B_QK_FULL + s), 2u * 8192u);
-        tma::load_3d(qraw, &m.q, 0, x.h, tok0, x.bar(B_QK_FULL + s));
-        tma::load_3d(qraw + 4096, &m.q, 64, x.h, tok0, x.bar(B_QK_FULL + s));
-        tma::load_3d(kraw, &m.k, 0, x.h, tok0, x.bar(B_QK_FULL + s));
-        tma::load_3d(kraw + 4096, &m.k, 64, x.h, tok0, x.bar(B_QK_FULL + s));
+        const uint32_t full = x.bar(B_QK_FULL + cq % R::NFULL);
+        tma::mbar_arrive_expect_tx(full, 2u * 8192u);
+        tma::load_tile(raw, &m.q, x.h, tok0, full);
+        tma::load_tile(raw + 8192, &m.k, x.h, tok0, full);
         cq++;
+        if (++sq == R::NQK) { sq = 0; pq ^= 1; }
         progressed = true;
       }
     }
     if (cg < n) {
       const int s = cg & 1;
       if (mbar_test_wait(x.bar(B_G_EMPTY + s), (uint32_t)(((cg >> 1) & 1) ^ 1))) {
-        uint8_t* raw = x.smem + OFF_RAW + s * RAW_STAGE;
         const int tok0 = (int)(x.t0 + (long long)cg * C);
-        tma::mbar_arrive_expect_tx(x.bar(B_G_FULL + s), FE == 1 ? 16384u : 8192u);
-        tma::load_3d(smem_u32(raw + RAW_G), &m.g, 0, x.h, tok0, x.bar(B_G_FULL + s));
+        const uint32_t full = x.bar(B_G_FULL + s);
+        tma::mbar_arrive_expect_tx(full, (uint32_t)R::G_BYTES);
+        tma::load_tile(smem_u32(x.smem + R::OFF_G + s * R::G_BYTES), &m.g, x.h, tok0, full);
         cg++;
         progressed = true;
       }
@@ -191,11 +211,9 @@ __device__ void role_loader(const ChunkParams& p, const TmaMaps& m, const Ctx& x
     if (cv < n) {
       const int s = cv & 1;
       if (mbar_test_wait(x.bar(B_V_EMPTY + s), (uint32_t)(((cv >> 1) & 1) ^ 1))) {
-        const uint32_t vdst = smem_u32(x.smem + OFF_CONS + s * CS_STAGE + CS_V);
         const int tok0 = (int)(x.t0 + (long long)cv * C);
         tma::mbar_arrive_expect_tx(x.bar(B_V_FULL + s), 8192u);
-        tma::load_3d(vdst, &m.v, 0, x.h, tok0, x.bar(B_V_FULL + s));
-        tma::load_3d(vdst + 4096, &m.v, 64, x.h, tok0, x.bar(B_V_FULL + s));
+        tma::load_tile(smem_u32(x.smem + s * STAGE + CS_V), &m.v, x.h, tok0, x.bar(B_V_FULL + s));
         cv++;
         progressed = true;
       }
@@ -214,7 +232,7 @@ __device__ void role_loader(const ChunkParams& p, const TmaMaps& m, const Ctx& x
       }
     }
   }
-  loader_drain(x.bars, x.abort_flag, cg, cq, (p.debug_flags & DBG_STALL_V_STREAM) ? 0 : cv);
+  loader_drain(x.bars, x.abort_flag, cg, cq, (p.debug_flags & DBG_STALL_V_STREAM) ? 0 : cv, R::NFULL);
 }
 
 template <int FE>
@@ -227,174 +245,225 @@ __device__ __forceinline__ float load_beta(const ChunkParams& p, const Ctx& x, i
 }
 
 // ------------------------------------------------------------------------------------------------ prep warps
+// Operand preparation.  A warp owns 16 channels of all 32 tokens, a lane four channels (its quad) of four tokens (its token
+// group): the cumulative decay then runs along the lanes of one warp and never leaves registers, so a chunk costs the group
+// ONE barrier (in front of the intra-chunk products, which contract over all channels).  Of the four tokens of a lane, token
+// (j ^ sw) comes j-th, sw = 0 or 2 by token group: with that order every 16- and 8-byte access to the swizzled tiles is free
+// of bank conflicts (the eight or sixteen lanes of one phase touch rows that differ in the swizzle bits), and the address of
+// step j is that of step 0 with j flipped into the row and chunk bits.
+// (A layout of four tokens x 128 channels per warp sent the cumulative sums through shared memory and two more barriers.)
 template <int FE>
 __device__ void role_prep(const ChunkParams& p, const Ctx& x, int grp, int ptid) {
   const int pw = ptid >> 5, lane = ptid & 31;
-  const int ch = ptid & 127, half = ptid >> 7;
-  const int s = grp;                                   // the group's raw and consumer stage
+  const int quad = lane & 3, tg = lane >> 2;
+  const int sw = ((tg ^ (tg >> 1)) & 1) << 1;
+  const int tok0 = 4 * tg + sw;                        // token of step j: tok0 ^ j
+  const bool first = tg < 4;                           // tokens 0-15
+  const int s = grp;                                   // the group's stage
   const int bar_id = 1 + grp;
-  float eA = 0.0f, dtb = 0.0f;
+  typedef Raw<FE> R;
+  uint8_t* st = x.smem + s * STAGE;
+  const uint8_t* g_tile = x.smem + R::OFF_G + s * R::G_BYTES;
+  float* norm = reinterpret_cast<float*>(x.smem + OFF_NORM) + s * 128;
+  int sq = grp, fq = grp;                              // q / k stage of the chunk, its full barrier and parity
+  uint32_t pq = 0;
+  // offsets of step 0 (step j: ^ j * 0x90 for rows of 128 bytes, ^ j * 0xa0 for kr)
+  const uint32_t off_f32 = (uint32_t)(tok0 * 128 + (((4 * (pw & 1) + quad) ^ (tok0 & 7)) << 4));
+  const uint32_t off_g = FE == 1 ? (uint32_t)((pw >> 1) * 4096) + off_f32 : 0u;
+  const uint32_t off_kd = (uint32_t)((pw >> 1) * 8192) + off_f32;
+  const uint32_t off_b16 = (uint32_t)((pw >> 2) * 4096 + tok0 * 128 + (((2 * (pw & 3) + (quad >> 1)) ^ (tok0 & 7)) << 4) + (quad & 1) * 8);
+  const uint32_t off_kr = (uint32_t)((pw >> 1) * 512 + tg * 2048 + sw * 128 + (((2 * (pw & 1) + (quad >> 1)) ^ sw) << 5) + (quad & 1) * 16);
+  float m1 = 0.0f, m0[4];
   if (FE == 0) {
-    eA = __expf(p.A_log[x.h]);
-    dtb = p.dt_bias[x.h * D + ch];
+    m1 = -LOG2E * __expf(p.A_log[x.h]);
+    const float* b = p.dt_bias + x.h * D + 16 * pw + 4 * quad;       // (any alignment)
+#pragma unroll
+    for (int i = 0; i < 4; i++) m0[i] = m1 * b[i];
   }
-  float* fr = reinterpret_cast<float*>(x.smem + OFF_FR) + grp * 3 * D;
-  float* fer = fr + D;
-  float* tot = fr + 2 * D;
-  uint8_t* raw = x.smem + OFF_RAW + s * RAW_STAGE;
-  uint8_t* cons = x.smem + OFF_CONS + s * CS_STAGE;
-  uint8_t* kis_tile = x.smem + OFF_KIS + grp * 8192;
-  float* Gsm = reinterpret_cast<float*>(raw + RAW_G);
-  float* beta_s = reinterpret_cast<float*>(x.smem + OFF_BETA) + s * 32;
+  const float scale = p.scale;
   volatile int* range_flag = reinterpret_cast<volatile int*>(x.smem + OFF_MISC + 12);
   float beta_next = (ptid < C && grp < x.nchunks) ? load_beta<FE>(p, x, grp, ptid) : 0.0f;   // one own chunk ahead
 #pragma unroll 1
   for (int c = grp; c < x.nchunks; c += PREP_GROUPS) {
     const uint32_t par = (uint32_t)((c >> 1) & 1);
     const int nvalid = min(C, x.len - c * C);
-    float* dec = reinterpret_cast<float*>(x.smem + OFF_DEC) + (c & 3) * D;
-    x.wait(B_G_FULL + s, par, E_PREP);
+    // alternates so that step C of the chunk before may still read the other half
+    float* beta_s = reinterpret_cast<float*>(x.smem + OFF_BETA) + (2 * s + (int)par) * 32;
+    uint8_t* qk = x.smem + R::OFF_QK + sq * 16384;       // q, then k
     PROF_BEGIN;
+    x.wait(B_G_FULL + s, par, E_PREP);
+    PROF_STAMP(2, 11);
 
-    // ---- A: gate activation + inclusive cumulative log2-decay; two threads per channel, 16 tokens each.
-    // Touches only prep-private scratch (the decay slot c & 3 was last read four chunks ago), so it runs while the
-    // tensor core still works on older chunks.
+    // ---- A: gate activation + cumulative log2-decay relative to r = the one after token 15 (tokens 0-15: own sum - r >= 0,
+    // tokens 16-31: their own partial sum <= 0)
+    float2 e[4][2], er[2], el[2];                        // exponents by step and channel pair; 2^r, 2^(G31 - r)
     {
-      float a[16];
+      float2 unit;
+      unit.x = unit.y = (FE == 1) ? LOG2E : p.lower_bound * LOG2E;
+      float2 a[4][2];
       if (FE == 1) {
-        const float* g = reinterpret_cast<const float*>(raw + RAW_G);
 #pragma unroll
-        for (int i = 0; i < 16; i++) a[i] = g[(16 * half + i) * D + ch];
+        for (int j = 0; j < 4; j++) {
+          const float4 f = *reinterpret_cast<const float4*>(g_tile + (off_g ^ (j * 0x90)));
+          a[j][0] = make_float2(f.x, f.y);
+          a[j][1] = make_float2(f.z, f.w);
+        }
       } else {
         // log2-decay = lower_bound log2(e) sigmoid(x), x = exp(A_log) (g + dt_bias); sigmoid(x) = 1 / (1 + 2^(-x log2 e))
         // with the exponent argument formed by one fused multiply-add per element
-        const __nv_bfloat16* g = reinterpret_cast<const __nv_bfloat16*>(raw + RAW_G);
-        const float m1 = -LOG2E * eA, m0 = m1 * dtb;
 #pragma unroll
-        for (int i = 0; i < 16; i++) a[i] = rcpf(1.0f + ex2f(fmaf(__bfloat162float(g[(16 * half + i) * D + ch]), m1, m0)));
-      }
-      if (nvalid < C) {                       // rows of the next sequence (last chunk only): no decay
-#pragma unroll
-        for (int i = 0; i < 16; i++)
-          if (16 * half + i >= nvalid) a[i] = 0.0f;
-      }
-      // inclusive cumulative sum in log2 units, the unit conversion fused into the additions
-      const float unit = (FE == 1) ? LOG2E : p.lower_bound * LOG2E;
-      a[0] *= unit;
-#pragma unroll
-      for (int i = 1; i < 16; i++) a[i] = fmaf(a[i], unit, a[i - 1]);
-      if (FE == 1) {
-        // fp32 gates are replaced in place by the thread that read them, so only the first-half sums cross threads:
-        // warp pw hands the sums of its 32 channels to warp pw + 4 through a barrier of their own.
-        if (half == 0) {
-          tot[ch] = a[15];
-          __syncwarp();
-          if (lane == 0) mbar_arrive(x.bar(B_TOT + 4 * grp + pw));
-        } else {
-          x.wait(B_TOT + 4 * grp + (pw - 4), par, E_PREP);
+        for (int j = 0; j < 4; j++) {
+          const uint2 f = *reinterpret_cast<const uint2*>(g_tile + (off_b16 ^ (j * 0x90)));
+          a[j][0] = make_float2(rcpf(1.0f + ex2f(fmaf(bf16_lo(f.x), m1, m0[0]))), rcpf(1.0f + ex2f(fmaf(bf16_hi(f.x), m1, m0[1]))));
+          a[j][1] = make_float2(rcpf(1.0f + ex2f(fmaf(bf16_lo(f.y), m1, m0[2]))), rcpf(1.0f + ex2f(fmaf(bf16_hi(f.y), m1, m0[3]))));
         }
-        PROF_STAMP(2, 10);
-        PROF_STAMP(2, 11);
-      } else {
-        if (half == 0) tot[ch] = a[15];
-        PROF_STAMP(2, 10);
-        named_bar_sync(bar_id, PREP_THREADS);   // all raw g values are in registers: the exponents may now overwrite the tile
-        PROF_STAMP(2, 11);
       }
-      // What step B needs is the exponent relative to r = G after token 15, clamped to the representable range:
-      // tokens 0-15 have G - r = own sum - r >= 0, tokens 16-31 have G - r = their own partial sum <= 0.
-      if (half == 1) {
-        const float r = tot[ch];
-        // Range of the primed operands: the largest exponents belong to token 0 (at most -r) and token 31 (a[15], the
-        // second half's own sum).  Beyond 2^126 they are clamped and the intra-chunk products of this chunk are no
-        // longer exact: report it.  (Checked here, by the threads that hold both numbers anyway, and reported by one
-        // lane per warp: these warps set the pace of the kernel, and a separate test in the first half of step A cost
-        // 2.7 % of it.)
-        if (__any_sync(0xffffffffu, fminf(r, a[15]) < -126.0f) && lane == 0) *range_flag = 1;
-        fer[ch] = ex2f(r);
-        dec[ch] = ex2f(a[15] + r);
-        tot[ch] = ex2f(a[15]);          // 2^(G31 - r), read back below as the kr factor
+      if (nvalid < C) {                                  // rows of the next sequence (last chunk only): no decay
 #pragma unroll
-        for (int i = 0; i < 16; i++) a[i] = fmaxf(a[i], -126.0f);
-      } else {
-        const float r = a[15];
+        for (int j = 0; j < 4; j++)
+          if ((tok0 ^ j) >= nvalid) a[j][0] = a[j][1] = make_float2(0.0f, 0.0f);
+      }
+      const bool p1 = (tg & 3) >= 1, p2 = (tg & 3) >= 2;
+      float2 own[2], oth[2];                             // sums over this lane's half of the chunk and over the other half
 #pragma unroll
-        for (int i = 0; i < 16; i++) a[i] = fminf(a[i] - r, 126.0f);
+      for (int i = 0; i < 2; i++) {
+        // sums inside the two token pairs, the unit conversion fused into the additions
+        e[0][i] = mul2(a[0][i], unit);
+        e[1][i] = fma2(a[1][i], unit, e[0][i]);
+        e[2][i] = mul2(a[2][i], unit);
+        e[3][i] = fma2(a[3][i], unit, e[2][i]);
+        const float2 sum = add2(e[1][i], e[3][i]);
+        // inclusive sum over the four token groups of the half
+        float2 inc = sum, t;
+        t.x = __shfl_up_sync(0xffffffffu, inc.x, 4);
+        t.y = __shfl_up_sync(0xffffffffu, inc.y, 4);
+        if (p1) inc = add2(inc, t);
+        t.x = __shfl_up_sync(0xffffffffu, inc.x, 8);
+        t.y = __shfl_up_sync(0xffffffffu, inc.y, 8);
+        if (p2) inc = add2(inc, t);
+        own[i].x = __shfl_sync(0xffffffffu, inc.x, (lane & 19) | 12);
+        own[i].y = __shfl_sync(0xffffffffu, inc.y, (lane & 19) | 12);
+        oth[i].x = __shfl_sync(0xffffffffu, inc.x, ((lane & 19) | 12) ^ 16);
+        oth[i].y = __shfl_sync(0xffffffffu, inc.y, ((lane & 19) | 12) ^ 16);
+        // what precedes this group in its half, less r in the first half; the later token pair of the group adds the earlier one
+        float2 base = make_float2(inc.x - sum.x, inc.y - sum.y);
+        if (first) base = make_float2(base.x - own[i].x, base.y - own[i].y);
+        const float2 zero = make_float2(0.0f, 0.0f);
+        const float2 b0 = add2(base, sw ? e[3][i] : zero), b1 = add2(base, sw ? zero : e[1][i]);
+        e[0][i] = add2(e[0][i], b0);
+        e[1][i] = add2(e[1][i], b0);
+        e[2][i] = add2(e[2][i], b1);
+        e[3][i] = add2(e[3][i], b1);
+      }
+      // The gates are in registers: the tile may be refilled.  Not right behind the loads: an arrival does not wait for loads
+      // in flight (they may sit behind hundreds of cycles of other traffic), only the arithmetic on their values does.
+      __syncwarp();
+      if (lane == 0) mbar_arrive(x.bar(B_G_EMPTY + s));
+      // Range of the primed operands: no exponent exceeds the decay of its half of the chunk.  Beyond 2^126 they are clamped
+      // and the intra-chunk products of this chunk are no longer exact: report it.
+      const float least = fminf(fminf(fminf(own[0].x, own[0].y), fminf(own[1].x, own[1].y)), fminf(fminf(oth[0].x, oth[0].y), fminf(oth[1].x, oth[1].y)));
+      if (__any_sync(0xffffffffu, least < -126.0f)) {
+        if (lane == 0) *range_flag = 1;
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+#pragma unroll
+          for (int i = 0; i < 2; i++)
+            e[j][i] = first ? make_float2(fminf(e[j][i].x, 126.0f), fminf(e[j][i].y, 126.0f)) : make_float2(fmaxf(e[j][i].x, -126.0f), fmaxf(e[j][i].y, -126.0f));
       }
 #pragma unroll
-      for (int i = 0; i < 16; i++) Gsm[(16 * half + i) * D + ch] = a[i];
+      for (int i = 0; i < 2; i++) {
+        const float2 r = first ? own[i] : oth[i], l = first ? oth[i] : own[i];
+        er[i] = make_float2(ex2f(r.x), ex2f(r.y));
+        el[i] = make_float2(ex2f(l.x), ex2f(l.y));
+      }
+      if (tg == 0) {                                     // 2^G31 (the decay slot c & 3 was last read four chunks ago)
+        const float2 d0 = mul2(er[0], el[0]), d1 = mul2(er[1], el[1]);
+        *reinterpret_cast<float4*>(x.smem + OFF_DEC + (c & 3) * (D * 4) + (16 * pw + 4 * quad) * 4) = make_float4(d0.x, d0.y, d1.x, d1.y);
+      }
     }
     PROF_STAMP(2, 12);
-    named_bar_sync(bar_id, PREP_THREADS);
-    PROF_STAMP(2, 26);
-    // Every warp of the group has left the previous chunk (step C reads beta_s), so beta may be replaced only now; step
-    // C of this chunk reads it after the next barrier.
     if (ptid < C) {
       beta_s[ptid] = beta_next;
       if (c + PREP_GROUPS < x.nchunks) beta_next = load_beta<FE>(p, x, c + PREP_GROUPS, ptid);
     }
 
-    // ---- B: L2 norm and decayed operand tiles; a warp owns 4 tokens, a lane 4 channels.  [kd ; qd] is written as
-    // soon as MMA1 of the chunk two back has read the stage; kr waits in registers until MMA3 has released the rest.
-    x.wait(B_QK_FULL + s, par, E_PREP);
+    // ---- B: L2 norm and decayed operand tiles.  [kd ; qd] is written as soon as MMA1 of the chunk two back has read the
+    // stage; kr waits in registers until MMA3 has released the rest.
+    float qinv = 1.0f, kinv = 1.0f;                      // of the token of step `quad`
+    x.wait(B_QK_FULL + fq, pq, E_PREP);
+    PROF_STAMP(2, 13);
+    if (FE == 0) {
+      // Square sums of the rows: the diagonal of rows x rows^T on mma.sync, whose B operand is the A operand's registers.
+      // Warp w takes the 16 rows (w & 1) of q (w & 2: of k) over half of the channels; exact products, fp32 sums.
+      const int row = 16 * (pw & 1) + (lane & 15);
+      const uint32_t tile = smem_u32(qk + ((pw & 2) ? 8192 : 0)) + (uint32_t)((pw >> 2) * 4096 + row * 128);
+      float d0[4] = {0.0f, 0.0f, 0.0f, 0.0f}, d1[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+      for (int kt = 0; kt < 4; kt++) {
+        uint32_t a[4];
+        ldmatrix_x4(a, tile + (uint32_t)(((2 * kt + (lane >> 4)) ^ (row & 7)) << 4));
+        mma_bf16(d0, a, a[0], a[2]);                     // columns = rows 0-7: diagonal in the first two registers
+        mma_bf16(d1, a, a[1], a[3]);                     // columns = rows 8-15: diagonal in the last two
+      }
+      if ((tg >> 1) == quad) {                           // columns 2 quad, 2 quad + 1 against row tg
+        float* n = norm + (pw >> 2) * 64 + ((pw & 2) ? 32 : 0) + 16 * (pw & 1) + tg;
+        n[0] = (tg & 1) ? d0[1] : d0[0];
+        n[8] = (tg & 1) ? d1[3] : d1[2];
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(x.bar(B_NORM + s));
+      x.wait(B_NORM + s, par, E_PREP);
+      const float* n = norm + (tok0 ^ quad);
+      qinv = rsqrtf(fmaxf(n[0] + n[64], 1e-12f));        // x / max(||x||, 1e-6)
+      kinv = rsqrtf(fmaxf(n[32] + n[96], 1e-12f));
+    }
     x.wait(B_KDQD_EMPTY + s, par ^ 1, E_PREP);
     PROF_STAMP(2, 14);
-    float krr[4][4];
+    float2 kr[4][2];
     {
-      const float4 er4 = *reinterpret_cast<const float4*>(fer + 4 * lane);
-      const float4 elr4 = *reinterpret_cast<const float4*>(tot + 4 * lane);
-      const float er[4] = {er4.x, er4.y, er4.z, er4.w};
-      const float elr[4] = {elr4.x, elr4.y, elr4.z, elr4.w};
+      const float2 sc2 = make_float2(scale, scale);
+      const float2 eq[2] = {mul2(er[0], sc2), mul2(er[1], sc2)};       // scale of q rides on 2^r here and on M below
 #pragma unroll
-      for (int tt = 0; tt < 4; tt++) {
-        const int tok = 4 * pw + tt;
-        const uint32_t off = rawtile_off(tok, 4 * lane);
-        uint2 q2 = *reinterpret_cast<const uint2*>(raw + RAW_Q + off);
-        uint2 k2 = *reinterpret_cast<const uint2*>(raw + RAW_K + off);
-        if (nvalid < C && tok >= nvalid) { q2 = make_uint2(0u, 0u); k2 = make_uint2(0u, 0u); }   // rows of the next sequence
-        const float qf[4] = {bf16_lo(q2.x), bf16_hi(q2.x), bf16_lo(q2.y), bf16_hi(q2.y)};
-        const float kf[4] = {bf16_lo(k2.x), bf16_hi(k2.x), bf16_lo(k2.y), bf16_hi(k2.y)};
-        float qinv = p.scale, kinv = 1.0f;
+      for (int j = 0; j < 4; j++) {
+        const uint32_t o = off_b16 ^ (j * 0x90);
+        uint2 q2 = *reinterpret_cast<const uint2*>(qk + o), k2 = *reinterpret_cast<const uint2*>(qk + 8192 + o);
+        if (nvalid < C && (tok0 ^ j) >= nvalid) { q2 = make_uint2(0u, 0u); k2 = make_uint2(0u, 0u); }   // rows of the next sequence
+        float2 qn[2] = {make_float2(bf16_lo(q2.x), bf16_hi(q2.x)), make_float2(bf16_lo(q2.y), bf16_hi(q2.y))};
+        float2 kn[2] = {make_float2(bf16_lo(k2.x), bf16_hi(k2.x)), make_float2(bf16_lo(k2.y), bf16_hi(k2.y))};
         if (FE == 0) {
-          float sq = qf[0] * qf[0] + qf[1] * qf[1] + qf[2] * qf[2] + qf[3] * qf[3];
-          float sk = kf[0] * kf[0] + kf[1] * kf[1] + kf[2] * kf[2] + kf[3] * kf[3];
+          const float qi = __shfl_sync(0xffffffffu, qinv, (lane & 28) | j), ki = __shfl_sync(0xffffffffu, kinv, (lane & 28) | j);
 #pragma unroll
-          for (int o = 16; o > 0; o >>= 1) {
-            sq += __shfl_xor_sync(0xffffffffu, sq, o);
-            sk += __shfl_xor_sync(0xffffffffu, sk, o);
+          for (int i = 0; i < 2; i++) {
+            qn[i] = mul2(qn[i], make_float2(qi, qi));
+            kn[i] = mul2(kn[i], make_float2(ki, ki));
           }
-          qinv = p.scale * rsqrtf(fmaxf(sq, 1e-12f));   // x / max(||x||, 1e-6)
-          kinv = rsqrtf(fmaxf(sk, 1e-12f));
         }
-        const float4 G4 = *reinterpret_cast<const float4*>(Gsm + tok * D + 4 * lane);
-        const float Gv[4] = {G4.x, G4.y, G4.z, G4.w};
-        float kds[4], qds[4], kis[4], kdt[4], qdt[4];
+        float2 kd[2], qd[2], ki[2], kt[2], qt[2];
 #pragma unroll
-        for (int j = 0; j < 4; j += 2) {               // channel pairs, packed fp32x2 arithmetic
-          const float e0 = Gv[j], e1 = Gv[j + 1];
-          const float2 E = make_float2(ex2f(e0), ex2f(e1)), Ei = make_float2(ex2f(-e0), ex2f(-e1));
-          float2 kn = make_float2(kf[j], kf[j + 1]);
-          if (FE == 0) kn = mul2(kn, make_float2(kinv, kinv));
-          const float2 qn = mul2(make_float2(qf[j], qf[j + 1]), make_float2(qinv, qinv));
-          const float2 kd2 = mul2(kn, E), qd2 = mul2(qn, E), ki2 = mul2(kn, Ei);
-          const float2 er2 = make_float2(er[j], er[j + 1]);
-          const float2 kt2 = mul2(kd2, er2), qt2 = mul2(qd2, er2), kr2 = mul2(ki2, make_float2(elr[j], elr[j + 1]));
-          kds[j] = kd2.x; kds[j + 1] = kd2.y; qds[j] = qd2.x; qds[j + 1] = qd2.y; kis[j] = ki2.x; kis[j + 1] = ki2.y;
-          kdt[j] = kt2.x; kdt[j + 1] = kt2.y; qdt[j] = qt2.x; qdt[j + 1] = qt2.y; krr[tt][j] = kr2.x; krr[tt][j + 1] = kr2.y;
+        for (int i = 0; i < 2; i++) {
+          const float2 E = make_float2(ex2f(e[j][i].x), ex2f(e[j][i].y)), Ei = make_float2(ex2f(-e[j][i].x), ex2f(-e[j][i].y));
+          kd[i] = mul2(kn[i], E);
+          qd[i] = mul2(qn[i], E);
+          ki[i] = mul2(kn[i], Ei);
+          kt[i] = mul2(kd[i], er[i]);
+          qt[i] = mul2(qd[i], eq[i]);
+          kr[j][i] = mul2(ki[i], el[i]);
         }
         // in place: the decayed bf16 tiles of the intra-chunk products replace the raw q / k tiles
-        *reinterpret_cast<uint2*>(raw + RAW_K + off) = make_uint2(pack_bf16(kds[0], kds[1]), pack_bf16(kds[2], kds[3]));
-        *reinterpret_cast<uint2*>(raw + RAW_Q + off) = make_uint2(pack_bf16(qds[0], qds[1]), pack_bf16(qds[2], qds[3]));
-        *reinterpret_cast<uint2*>(kis_tile + off) = make_uint2(pack_bf16(kis[0], kis[1]), pack_bf16(kis[2], kis[3]));
+        *reinterpret_cast<uint2*>(qk + 8192 + o) = make_uint2(pack_bf16(kd[0].x, kd[0].y), pack_bf16(kd[1].x, kd[1].y));
+        *reinterpret_cast<uint2*>(qk + o) = make_uint2(pack_bf16(qd[0].x, qd[0].y), pack_bf16(qd[1].x, qd[1].y));
+        *reinterpret_cast<uint2*>(st + KI + o) = make_uint2(pack_bf16(ki[0].x, ki[0].y), pack_bf16(ki[1].x, ki[1].y));
         // tf32 operands of the state products: [kd ; qd] K-major (row = token, 32 + token), kr MN-major
-        *reinterpret_cast<float4*>(cons + CS_KDQD + kmajor_f32_off(tok, 4 * lane, 8192)) = make_float4(kdt[0], kdt[1], kdt[2], kdt[3]);
-        *reinterpret_cast<float4*>(cons + CS_KDQD + kmajor_f32_off(32 + tok, 4 * lane, 8192)) = make_float4(qdt[0], qdt[1], qdt[2], qdt[3]);
+        const uint32_t f = off_kd ^ (j * 0x90);
+        *reinterpret_cast<float4*>(st + CS_KDQD + f) = make_float4(kt[0].x, kt[0].y, kt[1].x, kt[1].y);
+        *reinterpret_cast<float4*>(st + CS_KDQD + 4096 + f) = make_float4(qt[0].x, qt[0].y, qt[1].x, qt[1].y);
       }
     }
     PROF_STAMP(2, 27);
-    fence_proxy_async();                                  // this thread's reads / writes of the g region precede its refill
+    fence_proxy_async();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(x.bar(B_KDQD_FULL + s));
     named_bar_sync(bar_id, PREP_THREADS);
-    if (lane == 0) mbar_arrive(x.bar(B_G_EMPTY + s));     // the gate tile may be refilled: step C does not read it
     PROF_STAMP(2, 28);
 
     // ---- C: one 16x16 block of A = kd' ki'^T (warps 0-3) or M = qd' ki'^T (warps 4-7) per warp
@@ -408,8 +477,8 @@ __device__ void role_prep(const ChunkParams& p, const Ctx& x, int grp, int ptid)
 #pragma unroll
         for (int j = 0; j < 4; j++) acc[i][j] = 0.0f;
       if (!(rb == 0 && cb == 1)) {
-        const uint32_t a_tile = smem_u32(raw + (which ? RAW_Q : RAW_K));
-        const uint32_t b_tile = smem_u32(kis_tile);
+        const uint32_t a_tile = smem_u32(qk + (which ? 0 : 8192));
+        const uint32_t b_tile = smem_u32(st + KI);
         const int a_row = 16 * rb + (lane & 7) + ((lane >> 3) & 1) * 8;
         const int b_row = 16 * cb + 8 * (lane >> 4) + (lane & 7);
 #pragma unroll
@@ -421,16 +490,18 @@ __device__ void role_prep(const ChunkParams& p, const Ctx& x, int grp, int ptid)
           mma_bf16(acc[1], a, b[2], b[3]);
         }
       }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(x.bar(B_QK_EMPTY + sq));      // the q / k tiles are no longer read
       PROF_STAMP(2, 15);
       if (which == 0) {
         x.wait(B_L_EMPTY + s, par ^ 1, E_PREP);
-        float* Lsm = reinterpret_cast<float*>(x.smem + OFF_L) + s * 1024;
+        float* Lsm = reinterpret_cast<float*>(x.smem + OFF_L) + s * C * LS;
         const float b0 = beta_s[i0], b1 = beta_s[i1];
 #pragma unroll
         for (int nt = 0; nt < 2; nt++) {
           const int j = 16 * cb + 8 * nt + 2 * t;
-          *reinterpret_cast<float2*>(Lsm + i0 * C + j) = make_float2((j < i0) ? acc[nt][0] * b0 : 0.0f, (j + 1 < i0) ? acc[nt][1] * b0 : 0.0f);
-          *reinterpret_cast<float2*>(Lsm + i1 * C + j) = make_float2((j < i1) ? acc[nt][2] * b1 : 0.0f, (j + 1 < i1) ? acc[nt][3] * b1 : 0.0f);
+          *reinterpret_cast<float2*>(Lsm + i0 * LS + j) = make_float2((j < i0) ? acc[nt][0] * b0 : 0.0f, (j + 1 < i0) ? acc[nt][1] * b0 : 0.0f);
+          *reinterpret_cast<float2*>(Lsm + i1 * LS + j) = make_float2((j < i1) ? acc[nt][2] * b1 : 0.0f, (j + 1 < i1) ? acc[nt][3] * b1 : 0.0f);
         }
         if (pw == 0) reinterpret_cast<float*>(x.smem + OFF_LBETA)[s * 32 + lane] = beta_s[lane];
         __syncwarp();
@@ -441,141 +512,116 @@ __device__ void role_prep(const ChunkParams& p, const Ctx& x, int grp, int ptid)
       x.wait(B_CONS_EMPTY + s, par ^ 1, E_PREP);
       PROF_STAMP(2, 17);
 #pragma unroll
-      for (int tt = 0; tt < 4; tt++)
-        *reinterpret_cast<float4*>(cons + CS_KR + mnmajor_f32_off(4 * lane, 4 * pw + tt, 512, 2048)) =
-            make_float4(krr[tt][0], krr[tt][1], krr[tt][2], krr[tt][3]);
+      for (int j = 0; j < 4; j++)
+        *reinterpret_cast<float4*>(st + CS_KR + (off_kr ^ (j * 0xa0))) = make_float4(kr[j][0].x, kr[j][0].y, kr[j][1].x, kr[j][1].y);
       if (which == 1) {
 #pragma unroll
         for (int nt = 0; nt < 2; nt++) {
           const int j = 16 * cb + 8 * nt + 2 * t;
-          *reinterpret_cast<float2*>(cons + CS_M + kmajor_f32_off(i0, j, 0)) =
-              make_float2((j <= i0) ? acc[nt][0] : 0.0f, (j + 1 <= i0) ? acc[nt][1] : 0.0f);
-          *reinterpret_cast<float2*>(cons + CS_M + kmajor_f32_off(i1, j, 0)) =
-              make_float2((j <= i1) ? acc[nt][2] : 0.0f, (j + 1 <= i1) ? acc[nt][3] : 0.0f);
+          *reinterpret_cast<float2*>(st + CS_M + kmajor_f32_off(i0, j, 0)) =
+              make_float2((j <= i0) ? acc[nt][0] * scale : 0.0f, (j + 1 <= i0) ? acc[nt][1] * scale : 0.0f);
+          *reinterpret_cast<float2*>(st + CS_M + kmajor_f32_off(i1, j, 0)) =
+              make_float2((j <= i1) ? acc[nt][2] * scale : 0.0f, (j + 1 <= i1) ? acc[nt][3] * scale : 0.0f);
         }
       }
     }
     PROF_STAMP(2, 29);
     fence_proxy_async();
     __syncwarp();
-    if (lane == 0) {
-      mbar_arrive(x.bar(B_P1_FULL + s));
-      mbar_arrive(x.bar(B_QK_EMPTY + s));        // the q / k tiles are no longer read
-    }
+    if (lane == 0) mbar_arrive(x.bar(B_P1_FULL + s));
+    sq += PREP_GROUPS;
+    if (sq >= R::NQK) sq -= R::NQK;
+    fq += PREP_GROUPS;
+    if (fq >= R::NFULL) { fq -= R::NFULL; pq ^= 1; }
   }
 }
 
 // ------------------------------------------------------------------------------------------------ inverse warps
-// T = (I + L)^-1 for the strictly lower triangular fp32 L [32][32] of a chunk, in place in L's buffer, by one warp:
+// T = (I + L)^-1 for the strictly lower triangular fp32 L [32][32] of a chunk (row stride LS), by one warp:
 //   1. the two 16x16 diagonal blocks by forward substitution in fp32 registers, one half-warp per block, lane = column
-//      (16 dependent rows instead of 32);
-//   2. the off-diagonal block T10 = -T11 (L10 T00) as two 16x16x16 products on mma.sync (tf32 operands, fp32
-//      accumulation; T is consumed as a tf32 / bf16 tensor-core operand anyway).
-// Then Tb = T diag(beta) goes out as the tf32 and bf16 operand tiles of MMA2.
-__device__ __forceinline__ void mm16_tf32(float (&acc)[2][4], const float* A, const float* B, int lane) {
-  // acc[nt] (16 x 8) += A[16][16] * B[16][16], both row-major with a row stride of 32 floats
-  const int g = lane >> 2, t = lane & 3;
-#pragma unroll
-  for (int kt = 0; kt < 2; kt++) {
-    const uint32_t a[4] = {__float_as_uint(A[g * C + 8 * kt + t]), __float_as_uint(A[(g + 8) * C + 8 * kt + t]),
-                           __float_as_uint(A[g * C + 8 * kt + t + 4]), __float_as_uint(A[(g + 8) * C + 8 * kt + t + 4])};
-#pragma unroll
-    for (int nt = 0; nt < 2; nt++)
-      mma_tf32(acc[nt], a, __float_as_uint(B[(8 * kt + t) * C + 8 * nt + g]), __float_as_uint(B[(8 * kt + t + 4) * C + 8 * nt + g]));
-  }
-}
-
+//      (16 dependent rows instead of 32), in place;
+//   2. the off-diagonal block T10 = -(T11 L10) T00 as two 16x16x16 products on mma.sync (tf32 operands, fp32 accumulation; T
+//      is consumed as a tf32 / bf16 tensor-core operand anyway).  The accumulators of the first product are the A operand of
+//      the second as they lie: its contraction index is taken in the order 0, 2, 4, 6, 1, 3, 5, 7 on both sides.
+// Then Tb = T diag(beta) goes out as the tf32 and bf16 operand tiles of MMA2: the diagonal blocks row by row, T10 from the
+// accumulators; the upper right block is zeroed once.
 __device__ void role_inverse(const Ctx& x, int which, int lane) {
   const int blk = lane >> 4, cl = lane & 15;
   const int g = lane >> 2, t = lane & 3;
+  const int s = which;                                 // the warp's stage
+  float* Lsm = reinterpret_cast<float*>(x.smem + OFF_L) + s * C * LS;
+  const float* lbeta = reinterpret_cast<const float*>(x.smem + OFF_LBETA) + s * 32;
+  uint8_t* tb = x.smem + s * STAGE + CS_TB;
+  uint8_t* tbh = x.smem + OFF_TBH + s * 2048;
+  {
+    const uint4 z = make_uint4(0u, 0u, 0u, 0u);
+    *reinterpret_cast<uint4*>(tb + kmajor_f32_off(cl, 16 + 4 * blk, 0)) = z;
+    *reinterpret_cast<uint4*>(tb + kmajor_f32_off(cl, 24 + 4 * blk, 0)) = z;
+    *reinterpret_cast<uint4*>(tbh + kmajor_b16_sw64_off(cl, 16 + 8 * blk)) = z;
+  }
 #pragma unroll 1
   for (int c = which; c < x.nchunks; c += 2) {
-    const int s = c & 1;
     const uint32_t par = (uint32_t)((c >> 1) & 1);
-    // Everything that does not depend on this chunk's L comes first, while the warp would only wait for L anyway (the
-    // v tile and the release of the stage by MMA3 of the chunk two back are normally long there): after the inversion
-    // only the operand write-out remains between L and MMA2.
-    // The v tile of a partial last chunk holds another sequence's rows (or worse) past the end of the run: zero them
-    // so that they cannot poison MMA2 (their Tb columns are zero, but 0 * NaN is NaN).  This warp observes every
-    // phase of the v barrier of its stage, so the wait cannot be satisfied by an older phase, and MMA2 waits for this
-    // warp's INV_FULL arrival.
-    x.wait(B_V_FULL + s, par, E_INV);
-    {
-      const int nvalid = min(C, x.len - c * C);
-      if (nvalid < C) {
-        uint8_t* vt = x.smem + OFF_CONS + s * CS_STAGE + CS_V;
-        for (int i = lane; i < (C - nvalid) * 16; i += 32) {     // whole 128-byte lines of both 64-channel halves
-          const int row = nvalid + (i >> 4), piece = i & 15;
-          *reinterpret_cast<uint4*>(vt + (piece >> 3) * 4096 + row * 128 + (piece & 7) * 16) = make_uint4(0u, 0u, 0u, 0u);
-        }
-      }
-    }
-    x.wait(B_CONS_EMPTY + s, par ^ 1, E_INV);
     x.wait(B_L_FULL + s, par, E_INV);
-    float* Lsm = reinterpret_cast<float*>(x.smem + OFF_L) + s * 1024;
     PROF_BEGIN;
-    // ---- 1: diagonal blocks
+    // ---- 1: diagonal blocks.  L is zero on and above its diagonal, so a row takes whole groups of four columns.
     {
-      const float* Lb = Lsm + blk * 16 * C + blk * 16;
-      float Tc[16];
+      const float* Lb = Lsm + blk * 16 * LS + blk * 16;
+      float2 T[8];
 #pragma unroll
-      for (int i = 0; i < 16; i++) {
-        float a0 = 0.0f, a1 = 0.0f, a2 = 0.0f, a3 = 0.0f;
+      for (int i = 0; i < 8; i++) T[i] = make_float2(2 * i == cl ? 1.0f : 0.0f, 2 * i + 1 == cl ? 1.0f : 0.0f);
 #pragma unroll
-        for (int j = 0; j + 3 < i; j += 4) {
-          const float4 l4 = *reinterpret_cast<const float4*>(Lb + i * C + j);
-          a0 = fmaf(l4.x, Tc[j], a0);
-          a1 = fmaf(l4.y, Tc[j + 1], a1);
-          a2 = fmaf(l4.z, Tc[j + 2], a2);
-          a3 = fmaf(l4.w, Tc[j + 3], a3);
+      for (int i = 1; i < 16; i++) {
+        float2 a0 = make_float2(0.0f, 0.0f), a1 = a0;
+#pragma unroll
+        for (int j = 0; j < i; j += 4) {
+          const float4 l4 = *reinterpret_cast<const float4*>(Lb + i * LS + j);
+          a0 = fma2(make_float2(l4.x, l4.y), T[j / 2], a0);
+          a1 = fma2(make_float2(l4.z, l4.w), T[j / 2 + 1], a1);
         }
-#pragma unroll
-        for (int j = i & ~3; j < i; j++) a0 = fmaf(Lb[i * C + j], Tc[j], a0);
-        Tc[i] = ((i == cl) ? 1.0f : 0.0f) - ((a0 + a1) + (a2 + a3));
+        const float2 a = add2(a0, a1);
+        if (i & 1) T[i / 2].y -= a.x + a.y;
+        else T[i / 2].x -= a.x + a.y;
       }
       __syncwarp();                                   // every lane has read its diagonal block
-      float* Tb_ = Lsm + blk * 16 * C + blk * 16;
+      float* Tb_ = Lsm + blk * 16 * LS + blk * 16;
 #pragma unroll
-      for (int i = 0; i < 16; i++) Tb_[i * C + cl] = Tc[i];
+      for (int i = 0; i < 16; i++) Tb_[i * LS + cl] = (i & 1) ? T[i / 2].y : T[i / 2].x;
     }
+    PROF_STAMP(3, 25);
     __syncwarp();
-    // ---- 2: T10 = -T11 (L10 T00), in place in the (1,0) block
+    x.wait(B_CONS_EMPTY + s, par ^ 1, E_INV);         // MMA2 of the chunk two back has read Tb
+    // ---- 2: T10 = -(T11 L10) T00
+    float acc[2][4], out10[2][4];
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+#pragma unroll
+      for (int j = 0; j < 4; j++) acc[i][j] = out10[i][j] = 0.0f;
     {
-      float* L10 = Lsm + 16 * C;
-      float acc[2][4];
+      const float* T11 = Lsm + 16 * LS + 16;
+      const float* L10 = Lsm + 16 * LS;
 #pragma unroll
-      for (int i = 0; i < 2; i++)
+      for (int kt = 0; kt < 2; kt++) {
+        const uint32_t a[4] = {__float_as_uint(T11[g * LS + 8 * kt + t]), __float_as_uint(T11[(g + 8) * LS + 8 * kt + t]),
+                               __float_as_uint(T11[g * LS + 8 * kt + t + 4]), __float_as_uint(T11[(g + 8) * LS + 8 * kt + t + 4])};
 #pragma unroll
-        for (int j = 0; j < 4; j++) acc[i][j] = 0.0f;
-      mm16_tf32(acc, L10, Lsm, lane);                 // X = L10 T00
-      __syncwarp();                                   // L10 fully read
-#pragma unroll
-      for (int nt = 0; nt < 2; nt++) {
-        *reinterpret_cast<float2*>(L10 + g * C + 8 * nt + 2 * t) = make_float2(acc[nt][0], acc[nt][1]);
-        *reinterpret_cast<float2*>(L10 + (g + 8) * C + 8 * nt + 2 * t) = make_float2(acc[nt][2], acc[nt][3]);
-        acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.0f;
+        for (int nt = 0; nt < 2; nt++)
+          mma_tf32(acc[nt], a, __float_as_uint(L10[(8 * kt + t) * LS + 8 * nt + g]), __float_as_uint(L10[(8 * kt + t + 4) * LS + 8 * nt + g]));
       }
-      __syncwarp();
-      mm16_tf32(acc, Lsm + 16 * C + 16, L10, lane);   // T11 X
-      __syncwarp();                                   // X fully read
 #pragma unroll
-      for (int nt = 0; nt < 2; nt++) {
-        *reinterpret_cast<float2*>(L10 + g * C + 8 * nt + 2 * t) = make_float2(-acc[nt][0], -acc[nt][1]);
-        *reinterpret_cast<float2*>(L10 + (g + 8) * C + 8 * nt + 2 * t) = make_float2(-acc[nt][2], -acc[nt][3]);
+      for (int kt = 0; kt < 2; kt++) {
+        const uint32_t a[4] = {__float_as_uint(acc[kt][0]), __float_as_uint(acc[kt][2]), __float_as_uint(acc[kt][1]), __float_as_uint(acc[kt][3])};
+#pragma unroll
+        for (int nt = 0; nt < 2; nt++)
+          mma_tf32(out10[nt], a, __float_as_uint(Lsm[(8 * kt + 2 * t) * LS + 8 * nt + g]), __float_as_uint(Lsm[(8 * kt + 2 * t + 1) * LS + 8 * nt + g]));
       }
     }
-    __syncwarp();
-    const float* lbeta = reinterpret_cast<const float*>(x.smem + OFF_LBETA) + s * 32;
-    PROF_STAMP(3, 26);
-    uint8_t* tb = x.smem + OFF_CONS + s * CS_STAGE + CS_TB;
-    uint8_t* tbh = x.smem + OFF_TBH + s * 2048;
-    // Tb = T diag(beta): lane = row; eight columns (one 16-byte bf16 chunk, two 16-byte tf32 chunks) per step, the
-    // column group rotated by the lane so that the wide loads and stores of a quarter-warp spread over the banks.
+    // Tb, diagonal blocks: lane = row
 #pragma unroll
-    for (int jj = 0; jj < 4; jj++) {
-      const int c0 = 8 * ((jj + lane) & 3);
-      const float4 ta = *reinterpret_cast<const float4*>(Lsm + lane * C + c0);
-      const float4 tc = *reinterpret_cast<const float4*>(Lsm + lane * C + c0 + 4);
+    for (int q = 0; q < 2; q++) {
+      const int c0 = 16 * blk + 8 * q;
+      const float4 ta = *reinterpret_cast<const float4*>(Lsm + lane * LS + c0);
+      const float4 tc = *reinterpret_cast<const float4*>(Lsm + lane * LS + c0 + 4);
       const float4 ba = *reinterpret_cast<const float4*>(lbeta + c0);
       const float4 bb = *reinterpret_cast<const float4*>(lbeta + c0 + 4);
       const float4 va = make_float4(ta.x * ba.x, ta.y * ba.y, ta.z * ba.z, ta.w * ba.w);
@@ -585,12 +631,39 @@ __device__ void role_inverse(const Ctx& x, int which, int lane) {
       *reinterpret_cast<uint4*>(tbh + kmajor_b16_sw64_off(lane, c0)) =
           make_uint4(pack_bf16(va.x, va.y), pack_bf16(va.z, va.w), pack_bf16(vb.x, vb.y), pack_bf16(vb.z, vb.w));
     }
+    PROF_STAMP(3, 26);
+    // Tb, lower left block
+#pragma unroll
+    for (int nt = 0; nt < 2; nt++) {
+      const int j = 8 * nt + 2 * t;
+      const float2 b = *reinterpret_cast<const float2*>(lbeta + j);
+      const float2 lo = make_float2(-out10[nt][0] * b.x, -out10[nt][1] * b.y), hi = make_float2(-out10[nt][2] * b.x, -out10[nt][3] * b.y);
+      *reinterpret_cast<float2*>(tb + kmajor_f32_off(16 + g, j, 0)) = lo;
+      *reinterpret_cast<float2*>(tb + kmajor_f32_off(24 + g, j, 0)) = hi;
+      *reinterpret_cast<uint32_t*>(tbh + kmajor_b16_sw64_off(16 + g, j)) = pack_bf16(lo.x, lo.y);
+      *reinterpret_cast<uint32_t*>(tbh + kmajor_b16_sw64_off(24 + g, j)) = pack_bf16(hi.x, hi.y);
+    }
+    // The v tile of a partial last chunk holds another sequence's rows (or worse) past the end of the run: zero them
+    // so that they cannot poison MMA2 (their Tb columns are zero, but 0 * NaN is NaN).  MMA2 waits for this warp's
+    // INV_FULL arrival.  (The wait for MMA3 of the chunk two back above implies that the v barrier has completed that
+    // chunk's phase, so the wait here cannot be satisfied by an older one.)
+    if (x.len - c * C < C) {
+      x.wait(B_V_FULL + s, par, E_INV);
+      const int nvalid = x.len - c * C;
+      uint8_t* vt = x.smem + s * STAGE + CS_V;
+      for (int i = lane; i < (C - nvalid) * 16; i += 32) {     // whole 128-byte lines of both 64-channel halves
+        const int row = nvalid + (i >> 4), piece = i & 15;
+        *reinterpret_cast<uint4*>(vt + (piece >> 3) * 4096 + row * 128 + (piece & 7) * 16) = make_uint4(0u, 0u, 0u, 0u);
+      }
+    }
+    PROF_STAMP(3, 27);
     fence_proxy_async();
     __syncwarp();
     if (lane == 0) {
       mbar_arrive(x.bar(B_INV_FULL + s));
       mbar_arrive(x.bar(B_L_EMPTY + s));
     }
+    PROF_STAMP(3, 28);
   }
 }
 
@@ -612,23 +685,23 @@ __device__ void role_mma(const Ctx& x, uint32_t tmem_any, bool v_zero_any) {
   const uint32_t tS = tmem + TM_S;
   // Descriptors of stage 0, built once; a stage or K step only moves the 14-bit start-address field (units of 16
   // bytes), so every other descriptor is one 64-bit add away.
-  const uint64_t d_kdqd = make_sdesc(sb + OFF_CONS + CS_KDQD, 16, 1024, LAYOUT_SW128);
-  const uint64_t d_v = make_sdesc(sb + OFF_CONS + CS_V, 4096, 1024, LAYOUT_SW128);
+  const uint64_t d_kdqd = make_sdesc(sb + CS_KDQD, 16, 1024, LAYOUT_SW128);
+  const uint64_t d_v = make_sdesc(sb + CS_V, 4096, 1024, LAYOUT_SW128);
   const uint64_t d_tbh = make_sdesc(sb + OFF_TBH, 16, 512, LAYOUT_SW64);
-  const uint64_t d_tb = make_sdesc(sb + OFF_CONS + CS_TB, 16, 1024, LAYOUT_SW128);
-  const uint64_t d_kr = make_sdesc(sb + OFF_CONS + CS_KR, 512, 2048, LAYOUT_SW128_BASE32B);
-  const uint64_t d_m = make_sdesc(sb + OFF_CONS + CS_M, 16, 1024, LAYOUT_SW128);
+  const uint64_t d_tb = make_sdesc(sb + CS_TB, 16, 1024, LAYOUT_SW128);
+  const uint64_t d_kr = make_sdesc(sb + CS_KR, 512, 2048, LAYOUT_SW128_BASE32B);
+  const uint64_t d_m = make_sdesc(sb + CS_M, 16, 1024, LAYOUT_SW128);
   x.wait(B_S_READY, 0, E_MMA, 0);                  // initial state is in tensor memory
 #pragma unroll 1
   for (int c = 0; c < nchunks; c++) {
     const int s = c & 1;
     const uint32_t par = (uint32_t)((c >> 1) & 1);
-    const uint64_t so = (uint64_t)(s * (CS_STAGE >> 4));          // stage offset in the start-address field
+    const uint64_t so = (uint64_t)(s * (STAGE >> 4));          // stage offset in the start-address field
     const uint64_t so_tbh = (uint64_t)(s * (2048 >> 4));
     const uint32_t tWO = tmem + TM_WO + 64 * s;
     const uint32_t tU = tmem + TM_U + 32 * s;             // U alternates too: MMA2 of the next chunk never overwrites
                                                           // columns that MMA3 of this chunk may still be reading
-    x.wait(B_P1_FULL + s, par, E_MMA, 0);
+    x.wait(B_KDQD_FULL + s, par, E_MMA, 0);
     x.wait(B_O_EMPTY + s, par ^ 1, E_MMA, 0);
     tc_fence_after();
     PROF_BEGIN;
@@ -638,8 +711,8 @@ __device__ void role_mma(const Ctx& x, uint32_t tmem_any, bool v_zero_any) {
     mma_commit_pred(x.bar(B_MMA1_DONE), go);              // the tensor-memory warps may rescale the state
     mma_commit_pred(x.bar(B_KDQD_EMPTY + s), go);         // [kd ; qd] of this stage may be rewritten
     PROF_STAMP(4, 26);
+    x.wait(B_V_FULL + s, par, E_MMA, 0);                  // (over long before the inverse is; a wait costs some 150 cycles even so)
     x.wait(B_INV_FULL + s, par, E_MMA, 0);
-    x.wait(B_V_FULL + s, par, E_MMA, 0);
     tc_fence_after();
     if (!v_zero) {
 #pragma unroll
@@ -651,6 +724,8 @@ __device__ void role_mma(const Ctx& x, uint32_t tmem_any, bool v_zero_any) {
       mma_ts_tf32_pred(tU, tWO + 8 * ks, d_tb + so + (uint64_t)((ks * 32) >> 4), ID2B, (ks > 0) || !v_zero, go);
     PROF_STAMP(4, 27);
     mma_commit_pred(x.bar(B_V_EMPTY + s), go);            // the v tile may be refilled once MMA2 has read it
+    x.wait(B_P1_FULL + s, par, E_MMA, 0);                 // M and kr
+    tc_fence_after();
 #pragma unroll
     for (int ks = 0; ks < 4; ks++)                        // O += U M^T does not touch the state: issued before the wait
       mma_ts_tf32_pred(tWO + 32, tU + 8 * ks, d_m + so + (uint64_t)((ks * 32) >> 4), ID3B, 1, go);
@@ -866,12 +941,12 @@ __device__ void role_mma_dual(const Ctx& x, uint32_t tmem_any, bool v_zero_any) 
   constexpr uint32_t ID2B = make_idesc(FMT_TF32, 128, 32, 0, 0, 1);
   constexpr uint32_t ID3A = make_idesc(FMT_TF32, 128, 128, 0, 1, 0);
   constexpr uint32_t ID3B = make_idesc(FMT_TF32, 128, 32, 0, 0, 0);
-  const uint64_t d_kdqd = make_sdesc(sb + OFF_CONS + CS_KDQD, 16, 1024, LAYOUT_SW128);
-  const uint64_t d_v = make_sdesc(sb + OFF_CONS + CS_V, 4096, 1024, LAYOUT_SW128);
+  const uint64_t d_kdqd = make_sdesc(sb + CS_KDQD, 16, 1024, LAYOUT_SW128);
+  const uint64_t d_v = make_sdesc(sb + CS_V, 4096, 1024, LAYOUT_SW128);
   const uint64_t d_tbh = make_sdesc(sb + OFF_TBH, 16, 512, LAYOUT_SW64);
-  const uint64_t d_tb = make_sdesc(sb + OFF_CONS + CS_TB, 16, 1024, LAYOUT_SW128);
-  const uint64_t d_kr = make_sdesc(sb + OFF_CONS + CS_KR, 512, 2048, LAYOUT_SW128_BASE32B);
-  const uint64_t d_m = make_sdesc(sb + OFF_CONS + CS_M, 16, 1024, LAYOUT_SW128);
+  const uint64_t d_tb = make_sdesc(sb + CS_TB, 16, 1024, LAYOUT_SW128);
+  const uint64_t d_kr = make_sdesc(sb + CS_KR, 512, 2048, LAYOUT_SW128_BASE32B);
+  const uint64_t d_m = make_sdesc(sb + CS_M, 16, 1024, LAYOUT_SW128);
   const uint32_t tS0 = tmem + TD_S0, tS1 = tmem + TD_S1, tWO1 = tmem + TD_WO1;
   x.wait(B_S_READY, 0, E_MMA, 0);                  // initial states are in tensor memory
   x.wait(B_S_READY_T, 0, E_MMA, 0);
@@ -879,12 +954,12 @@ __device__ void role_mma_dual(const Ctx& x, uint32_t tmem_any, bool v_zero_any) 
   for (int c = 0; c < nchunks; c++) {
     const int s = c & 1;
     const uint32_t par = (uint32_t)((c >> 1) & 1), cpar = (uint32_t)(c & 1);
-    const uint64_t so = (uint64_t)(s * (CS_STAGE >> 4));
+    const uint64_t so = (uint64_t)(s * (STAGE >> 4));
     const uint64_t so_tbh = (uint64_t)(s * (2048 >> 4));
     const uint32_t tU0 = tmem + TD_U0 + 32 * s, tU1 = tmem + TD_U1 + 32 * s;
     // [W | O]: one buffer per chain (one phase per chunk), not per stage as in the single-chain role
     const uint32_t tWO0 = tmem + TD_WO0;
-    x.wait(B_P1_FULL + s, par, E_MMA, 0);
+    x.wait(B_KDQD_FULL + s, par, E_MMA, 0);
     x.wait(B_O_EMPTY + 0, cpar ^ 1, E_MMA, 0);
     tc_fence_after();
 #pragma unroll
@@ -898,8 +973,8 @@ __device__ void role_mma_dual(const Ctx& x, uint32_t tmem_any, bool v_zero_any) 
       mma_ts_tf32_pred(tWO1, tS1 + 8 * ks, d_kdqd + so + (uint64_t)(((ks >> 2) * 8192 + (ks & 3) * 32) >> 4), ID1, ks > 0, go);
     mma_commit_pred(x.bar(B_MMA1_DONE_T), go);
     mma_commit_pred(x.bar(B_KDQD_EMPTY + s), go);
+    x.wait(B_V_FULL + s, par, E_MMA, 0);                  // (over long before the inverse is; a wait costs some 150 cycles even so)
     x.wait(B_INV_FULL + s, par, E_MMA, 0);
-    x.wait(B_V_FULL + s, par, E_MMA, 0);
     tc_fence_after();
     if (!v_zero) {
 #pragma unroll
@@ -913,6 +988,8 @@ __device__ void role_mma_dual(const Ctx& x, uint32_t tmem_any, bool v_zero_any) 
     for (int ks = 0; ks < 4; ks++)                      // the transition chain has v = 0: U = - W Tb^T
       mma_ts_tf32_pred(tU1, tWO1 + 8 * ks, d_tb + so + (uint64_t)((ks * 32) >> 4), ID2B, ks > 0, go);
     mma_commit_pred(x.bar(B_V_EMPTY + s), go);
+    x.wait(B_P1_FULL + s, par, E_MMA, 0);
+    tc_fence_after();
 #pragma unroll
     for (int ks = 0; ks < 4; ks++)
       mma_ts_tf32_pred(tWO0 + 32, tU0 + 8 * ks, d_m + so + (uint64_t)((ks * 32) >> 4), ID3B, 1, go);
@@ -1120,7 +1197,7 @@ __global__ void __launch_bounds__(THREADS, 1) kda_chunk_umma_kernel(const ChunkP
     // forty serial initialisations.  Arrival counts: the eight warps of a preparation group or the eight tensor-memory
     // warps where a whole group signals, four for the L tile (half a group), one everywhere else.
     constexpr unsigned long long EIGHT = (3ull << B_G_EMPTY) | (3ull << B_P1_FULL) | (3ull << B_O_EMPTY) | (1ull << B_S_READY) |
-                                         (3ull << B_QK_EMPTY) | (1ull << B_S_READY_T);
+                                         (7ull << B_QK_EMPTY) | (1ull << B_S_READY_T) | (3ull << B_NORM) | (3ull << B_KDQD_FULL);
     static_assert(PREP_WARPS == 8, "arrival counts of the group barriers");
     for (int i = lane; i < NUM_BARS; i += 32) {
       int count = ((EIGHT >> i) & 1ull) ? 8 : 1;

@@ -1,0 +1,82 @@
+"""The stages of the fused chunk kernel: chunk counts around its rings of gate and q / k tiles, repeatability over fresh
+buffers (a tile refilled before its last reader shows here first), inputs of the least alignment that the call takes."""
+import random
+
+import pytest
+import torch
+
+import kda_oracle as ko
+from kda_testlib import DEV, D, cu_of, gold_plain, gold_raw, plain_on_device, to_dev
+
+pytestmark = pytest.mark.gpu
+
+# one to eight chunks, full and partial: the q / k ring has two or three stages, its barriers repeat after six chunks
+LENS = [1, 31, 32, 33, 64, 65, 96, 97, 128, 159, 161, 192, 223, 225, 256]
+
+
+@pytest.fixture(scope="module")
+def kda():
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+    import kda_b200
+    from kda_b200 import _cabi
+    _cabi.lib()
+    return kda_b200
+
+
+@pytest.mark.parametrize("order", [1, -1])
+def test_chunk_counts_raw(kda, order):
+    lens = LENS[::order]
+    inputs = ko.make_inputs_raw(2, lens, 31)
+    gold_o, gold_s, _ = gold_raw(inputs, lens)
+    out, fin = kda.run(*to_dev(inputs))
+    torch.cuda.synchronize()
+    ko.check_close(out.cpu(), gold_o, "output")
+    ko.check_close(fin.cpu(), gold_s, "final state")
+
+
+@pytest.mark.parametrize("g_mean", [0.0, 4.0])
+def test_chunk_counts_plain(kda, g_mean):
+    lens, H = LENS, 2
+    q, k, v, g, beta = plain_on_device(H, sum(lens), 32, g_mean)
+    init = torch.randn(len(lens), H, D, D, generator=torch.Generator(device=DEV).manual_seed(33), device=DEV) * 0.05
+    out, fin = kda.chunk_kda(q, k, v, g, beta, initial_state=init, output_final_state=True, cu_seqlens=cu_of(lens))
+    torch.cuda.synchronize()
+    gold_o, gold_s, _ = gold_plain(q.cpu(), k.cpu(), v.cpu(), g.cpu(), beta.cpu(), D ** -0.5, init.cpu(), lens)
+    ko.check_close(out.cpu(), gold_o, "output")
+    ko.check_close(fin.cpu(), gold_s, "final state")
+
+
+@pytest.mark.parametrize("raw", [True, False])
+def test_repeatable_over_fresh_buffers(kda, raw):
+    """About seven hundred ragged (sequence, head) tasks, five times over new tensors: the same bits."""
+    rng, H = random.Random(5), 32
+    lens = [rng.randint(1, 900) for _ in range(22)]
+    first = None
+    for _ in range(5):
+        q, k, v, g, beta = plain_on_device(H, sum(lens), 34)
+        init = torch.randn(len(lens), H, D, D, generator=torch.Generator(device=DEV).manual_seed(35), device=DEV) * 0.05
+        if raw:
+            res = kda.kda_prefill(q, k, v, g.to(torch.bfloat16), beta.to(torch.bfloat16), torch.zeros(H, device=DEV),
+                                  torch.zeros(H * D, device=DEV), init, cu_of(lens))
+        else:
+            res = kda.chunk_kda(q, k, v, g, beta, initial_state=init, output_final_state=True, cu_seqlens=cu_of(lens))
+        torch.cuda.synchronize()
+        res = [t.clone() for t in res]
+        if first is None:
+            first = res
+        assert all(torch.equal(a, b) for a, b in zip(res, first))
+
+
+@pytest.mark.parametrize("offset", [1, 2, 3])
+def test_dt_bias_of_any_alignment(kda, offset):
+    H, lens = 2, [70, 33]
+    inputs = to_dev(ko.make_inputs_raw(H, lens, 36))
+    ref = kda.run(*inputs)
+    buf = torch.empty(H * D + 4, device=DEV)
+    dt = buf[offset:offset + H * D]
+    dt.copy_(inputs[6])
+    inputs[6] = dt
+    res = kda.run(*inputs)
+    torch.cuda.synchronize()
+    assert all(torch.equal(a, b) for a, b in zip(res, ref))
