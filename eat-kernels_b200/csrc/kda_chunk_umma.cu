@@ -34,11 +34,12 @@
 //
 // What bounds it: with 28 warps every warp issues about one instruction per ten cycles, so a chunk lasts as long as the chain
 // [kd ; qd] free -> operand tiles -> intra-chunk products -> inverse -> MMA2 over the two stages; the tensor pipe needs 970
-// cycles of it (the MMAs of a chunk depend on one another and still issue back to back).  Cumulative decay in the lanes of one
-// warp, norms off that chain, an inverse that no longer waits for v and a third q / k stage for raw gates, whole calls on a
-// B200 before / after: 8 x 1024 tokens at 64 heads, raw 419 / 394 us; 1 x 8192 at 96 heads, raw 788 / 721; 1 x 32768 at 16
-// heads with checkpoints, raw 1022 / 953; 16 x U[128, 4096] at 32 heads, plain 573 / 553; 48 requests at 64 heads, plain
-// 1803 / 1711.
+// cycles of it (the MMAs of a chunk depend on one another and still issue back to back).  Whole calls on a B200, first with
+// cumulative sums through shared memory and an inverse that waited for v, then with sums in the lanes of one warp and a third
+// q / k stage for raw gates, now with the decay in the 16-lane form, paired output stores, beta fetched ahead and the norms in
+// front of the gates: 8 x 1024 tokens at 64 heads, raw 415 / 392 / 347 us; 1 x 8192 at 96 heads, raw 770 / 696 / 604; 1 x 32768
+// at 16 heads with checkpoints, raw 990 / 949 / 857; 16 x U[128, 4096] at 32 heads, plain 547 / 512 / 489; 48 requests at 64
+// heads, plain 1792 / 1667 / 1616; 512 x 64 tokens at 64 heads, plain 2347 / 2302 / 2312 (start and end of a task).
 #include "kda_common.cuh"
 #include "kda_plan.cuh"
 #include "kda_tma.cuh"
@@ -75,8 +76,7 @@ constexpr int LS = 40;                                        // row stride of L
 constexpr int OFF_L = OFF_TBH + 4096;                         // 2 x fp32 [32][LS]
 constexpr int OFF_DEC = OFF_L + 2 * C * LS * 4;               // 4 x 512 (a slot is rewritten four chunks later)
 constexpr int OFF_BETA = OFF_DEC + 2048;                      // beta of a chunk: 2 groups x 2 (alternating) x 128
-constexpr int OFF_LBETA = OFF_BETA + 512;                     // beta next to L: 2 x 128
-constexpr int OFF_BAR = OFF_LBETA + 256;                      // mbarriers
+constexpr int OFF_BAR = OFF_BETA + 512;                       // mbarriers
 constexpr int NUM_BARS = 43;
 constexpr int OFF_MISC = OFF_BAR + NUM_BARS * 8;              // +0 tmem slot, +8 abort code, +12 range flag, +16 wait limit (ns)
 constexpr int SMEM_BYTES = OFF_MISC + 64;
@@ -235,14 +235,16 @@ __device__ void role_loader(const ChunkParams& p, const TmaMaps& m, const Ctx& x
   loader_drain(x.bars, x.abort_flag, cg, cq, (p.debug_flags & DBG_STALL_V_STREAM) ? 0 : cv, R::NFULL);
 }
 
+// Beta of one token row of a chunk: the raw bits are fetched a chunk of the group ahead, the activation follows at their use
+// (right behind the load it would hold the warp for the latency of global memory).
 template <int FE>
-__device__ __forceinline__ float load_beta(const ChunkParams& p, const Ctx& x, int c, int row) {
-  const int nvalid = min(C, x.len - c * C);
-  if (row >= nvalid) return 0.0f;
-  const long long tok = x.t0 + (long long)c * C + row;
-  if (FE == 1) return reinterpret_cast<const float*>(p.beta)[tok * p.ldbeta + x.h];
-  return sigmoidf_rel(__bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p.beta)[tok * p.ldbeta + x.h]));
+__device__ __forceinline__ uint32_t load_beta(const ChunkParams& p, const Ctx& x, int c, int row) {
+  if (row >= x.len - c * C) return 0;
+  const long long at = (x.t0 + (long long)c * C + row) * p.ldbeta + x.h;
+  return FE == 1 ? reinterpret_cast<const uint32_t*>(p.beta)[at] : reinterpret_cast<const uint16_t*>(p.beta)[at];
 }
+template <int FE>
+__device__ __forceinline__ float activate_beta(uint32_t raw) { return FE == 1 ? __uint_as_float(raw) : sigmoidf_rel(bf16_lo(raw)); }
 
 // ------------------------------------------------------------------------------------------------ prep warps
 // Operand preparation.  A warp owns 16 channels of all 32 tokens, a lane four channels (its quad) of four tokens (its token
@@ -273,16 +275,25 @@ __device__ void role_prep(const ChunkParams& p, const Ctx& x, int grp, int ptid)
   const uint32_t off_kd = (uint32_t)((pw >> 1) * 8192) + off_f32;
   const uint32_t off_b16 = (uint32_t)((pw >> 2) * 4096 + tok0 * 128 + (((2 * (pw & 3) + (quad >> 1)) ^ (tok0 & 7)) << 4) + (quad & 1) * 8);
   const uint32_t off_kr = (uint32_t)((pw >> 1) * 512 + tg * 2048 + sw * 128 + (((2 * (pw & 1) + (quad >> 1)) ^ sw) << 5) + (quad & 1) * 16);
-  float m1 = 0.0f, m0[4];
+  float m1 = 0.0f;
+  float2 m0[2];
   if (FE == 0) {
     m1 = -LOG2E * __expf(p.A_log[x.h]);
     const float* b = p.dt_bias + x.h * D + 16 * pw + 4 * quad;       // (any alignment)
-#pragma unroll
-    for (int i = 0; i < 4; i++) m0[i] = m1 * b[i];
+    m0[0] = make_float2(m1 * b[0], m1 * b[1]);
+    m0[1] = make_float2(m1 * b[2], m1 * b[3]);
   }
   const float scale = p.scale;
   volatile int* range_flag = reinterpret_cast<volatile int*>(x.smem + OFF_MISC + 12);
-  float beta_next = (ptid < C && grp < x.nchunks) ? load_beta<FE>(p, x, grp, ptid) : 0.0f;   // one own chunk ahead
+  // Warps 1 and 5 have no block of the intra-chunk products: 5 looks after beta and zeroes, once, the upper right block of M.
+  const bool no_block = (pw & 3) == 1;
+  uint32_t beta_next = 0;                              // one own chunk ahead
+  if (pw == 5) {
+    if (grp < x.nchunks) beta_next = load_beta<FE>(p, x, grp, lane);
+    const uint4 z = make_uint4(0u, 0u, 0u, 0u);
+    *reinterpret_cast<uint4*>(st + CS_M + kmajor_f32_off(lane & 15, 16 + 4 * (lane >> 4), 0)) = z;
+    *reinterpret_cast<uint4*>(st + CS_M + kmajor_f32_off(lane & 15, 24 + 4 * (lane >> 4), 0)) = z;
+  }
 #pragma unroll 1
   for (int c = grp; c < x.nchunks; c += PREP_GROUPS) {
     const uint32_t par = (uint32_t)((c >> 1) & 1);
@@ -291,6 +302,29 @@ __device__ void role_prep(const ChunkParams& p, const Ctx& x, int grp, int ptid)
     float* beta_s = reinterpret_cast<float*>(x.smem + OFF_BETA) + (2 * s + (int)par) * 32;
     uint8_t* qk = x.smem + R::OFF_QK + sq * 16384;       // q, then k
     PROF_BEGIN;
+    if (FE == 0) {
+      x.wait(B_QK_FULL + fq, pq, E_PREP);
+      // Square sums of the rows: the diagonal of rows x rows^T on mma.sync, whose B operand is the A operand's registers.
+      // Warp w takes the 16 rows (w & 1) of q (w & 2: of k) over half of the channels; exact products, fp32 sums.  They
+      // travel to the other warps while the gates are worked out.
+      const int row = 16 * (pw & 1) + (lane & 15);
+      const uint32_t tile = smem_u32(qk + ((pw & 2) ? 8192 : 0)) + (uint32_t)((pw >> 2) * 4096 + row * 128);
+      float d0[4] = {0.0f, 0.0f, 0.0f, 0.0f}, d1[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+      for (int kt = 0; kt < 4; kt++) {
+        uint32_t a[4];
+        ldmatrix_x4(a, tile + (uint32_t)(((2 * kt + (lane >> 4)) ^ (row & 7)) << 4));
+        mma_bf16(d0, a, a[0], a[2]);                     // columns = rows 0-7: diagonal in the first two registers
+        mma_bf16(d1, a, a[1], a[3]);                     // columns = rows 8-15: diagonal in the last two
+      }
+      if ((tg >> 1) == quad) {                           // columns 2 quad, 2 quad + 1 against row tg
+        float* n = norm + (pw >> 2) * 64 + ((pw & 2) ? 32 : 0) + 16 * (pw & 1) + tg;
+        n[0] = (tg & 1) ? d0[1] : d0[0];
+        n[8] = (tg & 1) ? d1[3] : d1[2];
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(x.bar(B_NORM + s));
+    }
     x.wait(B_G_FULL + s, par, E_PREP);
     PROF_STAMP(2, 11);
 
@@ -314,8 +348,13 @@ __device__ void role_prep(const ChunkParams& p, const Ctx& x, int grp, int ptid)
 #pragma unroll
         for (int j = 0; j < 4; j++) {
           const uint2 f = *reinterpret_cast<const uint2*>(g_tile + (off_b16 ^ (j * 0x90)));
-          a[j][0] = make_float2(rcpf(1.0f + ex2f(fmaf(bf16_lo(f.x), m1, m0[0]))), rcpf(1.0f + ex2f(fmaf(bf16_hi(f.x), m1, m0[1]))));
-          a[j][1] = make_float2(rcpf(1.0f + ex2f(fmaf(bf16_lo(f.y), m1, m0[2]))), rcpf(1.0f + ex2f(fmaf(bf16_hi(f.y), m1, m0[3]))));
+#pragma unroll
+          for (int i = 0; i < 2; i++) {
+            const uint32_t w = i ? f.y : f.x;
+            const float2 y = fma2(make_float2(bf16_lo(w), bf16_hi(w)), make_float2(m1, m1), m0[i]);
+            const float2 d = add2(make_float2(ex2f(y.x), ex2f(y.y)), make_float2(1.0f, 1.0f));
+            a[j][i] = make_float2(rcpf(d.x), rcpf(d.y));
+          }
         }
       }
       if (nvalid < C) {                                  // rows of the next sequence (last chunk only): no decay
@@ -382,36 +421,17 @@ __device__ void role_prep(const ChunkParams& p, const Ctx& x, int grp, int ptid)
       }
     }
     PROF_STAMP(2, 12);
-    if (ptid < C) {
-      beta_s[ptid] = beta_next;
-      if (c + PREP_GROUPS < x.nchunks) beta_next = load_beta<FE>(p, x, c + PREP_GROUPS, ptid);
+    if (pw == 5) {
+      beta_s[lane] = lane < nvalid ? activate_beta<FE>(beta_next) : 0.0f;
+      if (c + PREP_GROUPS < x.nchunks) beta_next = load_beta<FE>(p, x, c + PREP_GROUPS, lane);
     }
 
     // ---- B: L2 norm and decayed operand tiles.  [kd ; qd] is written as soon as MMA1 of the chunk two back has read the
     // stage; kr waits in registers until MMA3 has released the rest.
     float qinv = 1.0f, kinv = 1.0f;                      // of the token of step `quad`
-    x.wait(B_QK_FULL + fq, pq, E_PREP);
+    if (FE == 1) x.wait(B_QK_FULL + fq, pq, E_PREP);
     PROF_STAMP(2, 13);
     if (FE == 0) {
-      // Square sums of the rows: the diagonal of rows x rows^T on mma.sync, whose B operand is the A operand's registers.
-      // Warp w takes the 16 rows (w & 1) of q (w & 2: of k) over half of the channels; exact products, fp32 sums.
-      const int row = 16 * (pw & 1) + (lane & 15);
-      const uint32_t tile = smem_u32(qk + ((pw & 2) ? 8192 : 0)) + (uint32_t)((pw >> 2) * 4096 + row * 128);
-      float d0[4] = {0.0f, 0.0f, 0.0f, 0.0f}, d1[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll
-      for (int kt = 0; kt < 4; kt++) {
-        uint32_t a[4];
-        ldmatrix_x4(a, tile + (uint32_t)(((2 * kt + (lane >> 4)) ^ (row & 7)) << 4));
-        mma_bf16(d0, a, a[0], a[2]);                     // columns = rows 0-7: diagonal in the first two registers
-        mma_bf16(d1, a, a[1], a[3]);                     // columns = rows 8-15: diagonal in the last two
-      }
-      if ((tg >> 1) == quad) {                           // columns 2 quad, 2 quad + 1 against row tg
-        float* n = norm + (pw >> 2) * 64 + ((pw & 2) ? 32 : 0) + 16 * (pw & 1) + tg;
-        n[0] = (tg & 1) ? d0[1] : d0[0];
-        n[8] = (tg & 1) ? d1[3] : d1[2];
-      }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(x.bar(B_NORM + s));
       x.wait(B_NORM + s, par, E_PREP);
       const float* n = norm + (tok0 ^ quad);
       qinv = rsqrtf(fmaxf(n[0] + n[64], 1e-12f));        // x / max(||x||, 1e-6)
@@ -476,34 +496,50 @@ __device__ void role_prep(const ChunkParams& p, const Ctx& x, int grp, int ptid)
       for (int i = 0; i < 2; i++)
 #pragma unroll
         for (int j = 0; j < 4; j++) acc[i][j] = 0.0f;
-      if (!(rb == 0 && cb == 1)) {
-        const uint32_t a_tile = smem_u32(qk + (which ? 0 : 8192));
-        const uint32_t b_tile = smem_u32(st + KI);
-        const int a_row = 16 * rb + (lane & 7) + ((lane >> 3) & 1) * 8;
-        const int b_row = 16 * cb + 8 * (lane >> 4) + (lane & 7);
+      if (!no_block) {
+        // K step kt reads 16-byte chunks 2 kt, 2 kt + 1 of a row: two bits of the swizzled address flipped, then the second block
+        const uint32_t a_addr = smem_u32(qk + (which ? 0 : 8192)) + rawtile_off(16 * rb + (lane & 7) + ((lane >> 3) & 1) * 8, (lane >> 4) * 8);
+        const uint32_t b_addr = smem_u32(st + KI) + rawtile_off(16 * cb + 8 * (lane >> 4) + (lane & 7), ((lane >> 3) & 1) * 8);
 #pragma unroll
-        for (int kt = 0; kt < 8; kt++) {
-          uint32_t a[4], b[4];
-          ldmatrix_x4(a, a_tile + rawtile_off(a_row, (2 * kt + (lane >> 4)) * 8));
-          ldmatrix_x4(b, b_tile + rawtile_off(b_row, (2 * kt + ((lane >> 3) & 1)) * 8));
-          mma_bf16(acc[0], a, b[0], b[1]);
-          mma_bf16(acc[1], a, b[2], b[3]);
+        for (int kh = 0; kh < 8; kh += 2) {
+          uint32_t a[2][4], b[2][4];
+#pragma unroll
+          for (int i = 0; i < 2; i++) {
+            const int kt = kh + i;
+            ldmatrix_x4(a[i], (a_addr ^ ((kt & 3) << 5)) + (kt >> 2) * 4096);
+            ldmatrix_x4(b[i], (b_addr ^ ((kt & 3) << 5)) + (kt >> 2) * 4096);
+          }
+#pragma unroll
+          for (int i = 0; i < 2; i++) {
+            mma_bf16(acc[0], a[i], b[i][0], b[i][1]);
+            mma_bf16(acc[1], a[i], b[i][2], b[i][3]);
+          }
         }
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(x.bar(B_QK_EMPTY + sq));      // the q / k tiles are no longer read
+      if (rb == cb) {                                          // diagonal block: strictly lower for A, lower for M
+        const int m = g + which;
+#pragma unroll
+        for (int nt = 0; nt < 2; nt++) {
+          const int j = 8 * nt + 2 * t;
+          acc[nt][0] = j < m ? acc[nt][0] : 0.0f;
+          acc[nt][1] = j + 1 < m ? acc[nt][1] : 0.0f;
+          acc[nt][2] = j < m + 8 ? acc[nt][2] : 0.0f;
+          acc[nt][3] = j + 1 < m + 8 ? acc[nt][3] : 0.0f;
+        }
+      }
       PROF_STAMP(2, 15);
-      if (which == 0) {
+      if (which == 0 && !no_block) {
         x.wait(B_L_EMPTY + s, par ^ 1, E_PREP);
         float* Lsm = reinterpret_cast<float*>(x.smem + OFF_L) + s * C * LS;
         const float b0 = beta_s[i0], b1 = beta_s[i1];
 #pragma unroll
         for (int nt = 0; nt < 2; nt++) {
           const int j = 16 * cb + 8 * nt + 2 * t;
-          *reinterpret_cast<float2*>(Lsm + i0 * LS + j) = make_float2((j < i0) ? acc[nt][0] * b0 : 0.0f, (j + 1 < i0) ? acc[nt][1] * b0 : 0.0f);
-          *reinterpret_cast<float2*>(Lsm + i1 * LS + j) = make_float2((j < i1) ? acc[nt][2] * b1 : 0.0f, (j + 1 < i1) ? acc[nt][3] * b1 : 0.0f);
+          *reinterpret_cast<float2*>(Lsm + i0 * LS + j) = make_float2(acc[nt][0] * b0, acc[nt][1] * b0);
+          *reinterpret_cast<float2*>(Lsm + i1 * LS + j) = make_float2(acc[nt][2] * b1, acc[nt][3] * b1);
         }
-        if (pw == 0) reinterpret_cast<float*>(x.smem + OFF_LBETA)[s * 32 + lane] = beta_s[lane];
         __syncwarp();
         if (lane == 0) mbar_arrive(x.bar(B_L_FULL + s));      // the inverse of this chunk may start
       }
@@ -514,14 +550,12 @@ __device__ void role_prep(const ChunkParams& p, const Ctx& x, int grp, int ptid)
 #pragma unroll
       for (int j = 0; j < 4; j++)
         *reinterpret_cast<float4*>(st + CS_KR + (off_kr ^ (j * 0xa0))) = make_float4(kr[j][0].x, kr[j][0].y, kr[j][1].x, kr[j][1].y);
-      if (which == 1) {
+      if (which == 1 && !no_block) {
 #pragma unroll
         for (int nt = 0; nt < 2; nt++) {
           const int j = 16 * cb + 8 * nt + 2 * t;
-          *reinterpret_cast<float2*>(st + CS_M + kmajor_f32_off(i0, j, 0)) =
-              make_float2((j <= i0) ? acc[nt][0] * scale : 0.0f, (j + 1 <= i0) ? acc[nt][1] * scale : 0.0f);
-          *reinterpret_cast<float2*>(st + CS_M + kmajor_f32_off(i1, j, 0)) =
-              make_float2((j <= i1) ? acc[nt][2] * scale : 0.0f, (j + 1 <= i1) ? acc[nt][3] * scale : 0.0f);
+          *reinterpret_cast<float2*>(st + CS_M + kmajor_f32_off(i0, j, 0)) = make_float2(acc[nt][0] * scale, acc[nt][1] * scale);
+          *reinterpret_cast<float2*>(st + CS_M + kmajor_f32_off(i1, j, 0)) = make_float2(acc[nt][2] * scale, acc[nt][3] * scale);
         }
       }
     }
@@ -550,7 +584,6 @@ __device__ void role_inverse(const Ctx& x, int which, int lane) {
   const int g = lane >> 2, t = lane & 3;
   const int s = which;                                 // the warp's stage
   float* Lsm = reinterpret_cast<float*>(x.smem + OFF_L) + s * C * LS;
-  const float* lbeta = reinterpret_cast<const float*>(x.smem + OFF_LBETA) + s * 32;
   uint8_t* tb = x.smem + s * STAGE + CS_TB;
   uint8_t* tbh = x.smem + OFF_TBH + s * 2048;
   {
@@ -563,6 +596,8 @@ __device__ void role_inverse(const Ctx& x, int which, int lane) {
   for (int c = which; c < x.nchunks; c += 2) {
     const uint32_t par = (uint32_t)((c >> 1) & 1);
     x.wait(B_L_FULL + s, par, E_INV);
+    // (beta of this chunk is replaced four chunks on, behind MMA3 of this one)
+    const float* lbeta = reinterpret_cast<const float*>(x.smem + OFF_BETA) + (2 * s + (int)par) * 32;
     PROF_BEGIN;
     // ---- 1: diagonal blocks.  L is zero on and above its diagonal, so a row takes whole groups of four columns.
     {
@@ -793,16 +828,40 @@ __device__ __noinline__ void store_state_rows(uint32_t tS, float* dst, void* ck,
   }
 }
 
-// r[i] <- r[i] * d[i] for 16 consecutive state columns (d in shared memory, 16-byte aligned)
-__device__ __forceinline__ void scale16(uint32_t (&r)[16], const float* d) {
+// Decay St <- St diag(d) of a warp's 32 value rows x 64 state columns (at tS), on the serial chain MMA1 -> decay -> MMA3 ->
+// MMA1 of the next chunk.  In the 16-lane form a thread holds columns 8 i + 2 (lane % 4), + 1 of every group of eight, so it
+// needs 16 of the 64 factors (eight 8-byte loads; the 32-lane form takes sixteen 16-byte loads, all lanes the same).  Four
+// pieces of 16 rows x 32 columns, the tensor-memory load of a piece in flight while the one before is scaled and stored.
+__device__ __forceinline__ void scale_piece(uint32_t (&r)[16], const float2* d) {
 #pragma unroll
-  for (int i = 0; i < 4; i++) {
-    const float4 d4 = *reinterpret_cast<const float4*>(d + 4 * i);
-    const float2 lo = mul2(make_float2(__uint_as_float(r[4 * i]), __uint_as_float(r[4 * i + 1])), make_float2(d4.x, d4.y));
-    const float2 hi = mul2(make_float2(__uint_as_float(r[4 * i + 2]), __uint_as_float(r[4 * i + 3])), make_float2(d4.z, d4.w));
-    r[4 * i] = __float_as_uint(lo.x); r[4 * i + 1] = __float_as_uint(lo.y);
-    r[4 * i + 2] = __float_as_uint(hi.x); r[4 * i + 3] = __float_as_uint(hi.y);
+  for (int i = 0; i < 8; i++) {
+    const float2 v = mul2(make_float2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1])), d[i >> 1]);
+    r[2 * i] = __float_as_uint(v.x); r[2 * i + 1] = __float_as_uint(v.y);
   }
+}
+__device__ __forceinline__ void decay64(uint32_t tS, const float* dcol, int lane) {
+  constexpr uint32_t ROWS16 = 16u << 16;
+  uint32_t a[16], b[16];
+  float2 d[8];
+  tmem_ld16x32(tS, a);
+#pragma unroll
+  for (int i = 0; i < 8; i++) d[i] = *reinterpret_cast<const float2*>(dcol + 8 * i + 2 * (lane & 3));
+  tmem_wait_ld();
+  tmem_ld16x32(tS + 32, b);
+  scale_piece(a, d);
+  tmem_st16x32(tS, a);
+  tmem_wait_ld();
+  tmem_ld16x32(tS + ROWS16, a);
+  scale_piece(b, d + 4);
+  tmem_st16x32(tS + 32, b);
+  tmem_wait_ld();
+  tmem_ld16x32(tS + ROWS16 + 32, b);
+  scale_piece(a, d);
+  tmem_st16x32(tS + ROWS16, a);
+  tmem_wait_ld();
+  scale_piece(b, d + 4);
+  tmem_st16x32(tS + ROWS16 + 32, b);
+  tmem_wait_st();
 }
 
 // Eight warps own the tensor-memory traffic that goes through registers: warp (quarter q, half hf) serves the 32
@@ -846,55 +905,45 @@ __device__ void role_tmem(const ChunkParams& p, const Task& task, const Ctx& x, 
   __syncwarp();
   if (lane == 0) mbar_arrive(x.bar(B_S_READY));
 
-  __nv_bfloat16* obase = ((task.flags & TF_OUT_AUX) ? p.out_aux : p.out) + (long long)x.h * D + v;
+  // Output: the two lanes of a pair exchange halves, so that a lane stores two neighbouring values of one token (even lanes
+  // the even tokens) instead of one value of every token.
+  const bool odd = lane & 1;
+  const bool write_out = !(task.flags & TF_NO_OUT);
+  const long long ldo = p.ldo;
+  __nv_bfloat16* orow = ((task.flags & TF_OUT_AUX) ? p.out_aux : p.out) + (x.t0 + 16 * hf + (int)odd) * ldo + (long long)x.h * D + (v & ~1);
+  const uint32_t sel = odd ? 0x3276u : 0x5410u;          // (own, other) packed token pairs -> this lane's token, lower value first
+  int ck_left = (task.ck != nullptr && p.ck_every_chunks > 0) ? 0 : 0x7fffffff;     // chunks to the next checkpoint row
+  const int nchunks = x.nchunks;
 #pragma unroll 1
-  for (int c = 0; c <= x.nchunks; c++) {
+  for (int c = 0; c <= nchunks; c++, ck_left--, orow += C * ldo) {
+    const int s = c & 1;
+    const uint32_t par = (uint32_t)((c >> 1) & 1);
+    const bool last = c == nchunks;
     x.wait(B_MMA1_DONE, (uint32_t)(c & 1), E_SCALE);
     tc_fence_after();
-    const bool last = c == x.nchunks;
-    const bool ck = !last && task.ck != nullptr && p.ck_every_chunks > 0 && (c % p.ck_every_chunks) == 0;
-    const float* dec = reinterpret_cast<const float*>(x.smem + OFF_DEC) + (c & 3) * D;
-    long long ck_off = 0;
-    if (ck) ck_off = (long long)(c / p.ck_every_chunks) * p.ck_row_stride + (long long)x.h * STATE_ELEMS;
     // Checkpoint rows and the final state leave tensor memory through an out-of-line routine, so that their register
     // needs do not weigh on the per-chunk path below.
+    const bool ck = ck_left == 0 && !last;
     if (ck || last) {
       float* dst = (last && task.dst != nullptr) ? task.dst + (size_t)x.h * STATE_ELEMS : nullptr;
       void* ckp = nullptr;
-      if (ck) ckp = p.ck_is_bf16 ? static_cast<void*>(reinterpret_cast<__nv_bfloat16*>(task.ck) + ck_off)
-                                 : static_cast<void*>(reinterpret_cast<float*>(task.ck) + ck_off);
+      if (ck) {
+        const long long ck_off = (long long)(c / p.ck_every_chunks) * p.ck_row_stride + (long long)x.h * STATE_ELEMS;
+        ckp = p.ck_is_bf16 ? static_cast<void*>(reinterpret_cast<__nv_bfloat16*>(task.ck) + ck_off)
+                           : static_cast<void*>(reinterpret_cast<float*>(task.ck) + ck_off);
+        ck_left = p.ck_every_chunks;
+      }
       if (KF && (task.flags & TF_DST_VF)) store_state_rows<0>(tS, dst, ckp, p.ck_is_bf16, v, hf);   // transition maps
       else store_state_rows<KF>(tS, dst, ckp, p.ck_is_bf16, v, hf);
     }
     if (last) break;
-    {
-      // The decay sits on the serial chain MMA1 -> decay -> MMA3 -> MMA1 of the next chunk: four 16-column pieces,
-      // the tensor-memory load of a piece in flight while the previous one is scaled and stored.
-      const float* dcol = dec + 64 * hf;
-      uint32_t a[16], b[16], e[16];
-      tmem_ld16(tS, a);
-      tmem_ld16(tS + 16, b);
-      tmem_wait_ld();
-      scale16(a, dcol);
-      tmem_st16(tS, a);
-      tmem_ld16(tS + 32, e);
-      scale16(b, dcol + 16);
-      tmem_st16(tS + 16, b);
-      tmem_ld16(tS + 48, a);
-      tmem_wait_ld();
-      scale16(e, dcol + 32);
-      tmem_st16(tS + 32, e);
-      scale16(a, dcol + 48);
-      tmem_st16(tS + 48, a);
-    }
-    tmem_wait_st();
+    decay64(tS, reinterpret_cast<const float*>(x.smem + OFF_DEC) + (c & 3) * D + 64 * hf, lane);
     tc_fence_before();
     __syncwarp();
     if (lane == 0) mbar_arrive(x.bar(B_S_READY));
 
     // ---- output rows of this chunk
-    const int s = c & 1;
-    x.wait(B_O_FULL + s, (uint32_t)((c >> 1) & 1), E_EPI);
+    x.wait(B_O_FULL + s, par, E_EPI);
     tc_fence_after();
     uint32_t o[16];
     tmem_ld16(tmem + TM_WO + 64 * s + 32 + 16 * hf + lane_base, o);
@@ -902,16 +951,21 @@ __device__ void role_tmem(const ChunkParams& p, const Task& task, const Ctx& x, 
     tc_fence_before();
     __syncwarp();
     if (lane == 0) mbar_arrive(x.bar(B_O_EMPTY + s));
-    if (!(task.flags & TF_NO_OUT)) {
-      const int nvalid = min(C, x.len - c * C);
-      __nv_bfloat16* orow = obase + (x.t0 + (long long)c * C + 16 * hf) * p.ldo;
-      if (nvalid == C) {
+    if (write_out) {
+      uint32_t w[8];
 #pragma unroll
-        for (int i = 0; i < 16; i++) orow[(long long)i * p.ldo] = __float2bfloat16_rn(__uint_as_float(o[i]));
+      for (int i = 0; i < 8; i++) {
+        const uint32_t own = pack_bf16(__uint_as_float(o[2 * i]), __uint_as_float(o[2 * i + 1]));
+        w[i] = __byte_perm(own, __shfl_xor_sync(0xffffffffu, own, 1), sel);
+      }
+      const int left = x.len - c * C - 16 * hf - (int)odd;     // tokens of this run from this lane's first one on
+      if (x.len - c * C >= C) {
+#pragma unroll
+        for (int i = 0; i < 8; i++) *reinterpret_cast<uint32_t*>(orow + (long long)(2 * i) * ldo) = w[i];
       } else {
 #pragma unroll
-        for (int i = 0; i < 16; i++)
-          if (16 * hf + i < nvalid) orow[(long long)i * p.ldo] = __float2bfloat16_rn(__uint_as_float(o[i]));
+        for (int i = 0; i < 8; i++)
+          if (2 * i < left) *reinterpret_cast<uint32_t*>(orow + (long long)(2 * i) * ldo) = w[i];
       }
     }
   }
@@ -1016,27 +1070,6 @@ __device__ void role_mma_dual(const Ctx& x, uint32_t tmem_any, bool v_zero_any) 
   if (!mbar_wait_drain(x.bar(B_DRAIN), 0, x.abort_flag)) atomicCAS(const_cast<int*>(x.abort_flag), 0, E_DRAIN + B_DRAIN);
 }
 
-// St <- St diag(d) for this warp's 64 state columns (four 16-column pieces, the load of one in flight while the
-// previous one is scaled and stored)
-__device__ __forceinline__ void decay64(uint32_t tS, const float* dcol) {
-  uint32_t a[16], b[16], e[16];
-  tmem_ld16(tS, a);
-  tmem_ld16(tS + 16, b);
-  tmem_wait_ld();
-  scale16(a, dcol);
-  tmem_st16(tS, a);
-  tmem_ld16(tS + 32, e);
-  scale16(b, dcol + 16);
-  tmem_st16(tS + 16, b);
-  tmem_ld16(tS + 48, a);
-  tmem_wait_ld();
-  scale16(e, dcol + 32);
-  tmem_st16(tS + 32, e);
-  scale16(a, dcol + 48);
-  tmem_st16(tS + 48, a);
-  tmem_wait_st();
-}
-
 template <int KF>
 __device__ void role_tmem_dual(const ChunkParams& p, const Task& task, const Ctx& x, uint32_t tmem, int quarter, int hf, int lane) {
   const int v = 32 * quarter + lane;
@@ -1099,7 +1132,7 @@ __device__ void role_tmem_dual(const ChunkParams& p, const Task& task, const Ctx
           else store_state_rows<KF>(tS, dst, nullptr, 0, v, hf);
         }
       } else {
-        decay64(tS, dcol);
+        decay64(tS, dcol, lane);
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(x.bar(ch ? B_S_READY_T : B_S_READY));
@@ -1195,13 +1228,13 @@ __global__ void __launch_bounds__(THREADS, 1) kda_chunk_umma_kernel(const ChunkP
   if (warp == W_INV0) {
     // One lane per barrier (the issuer warp allocates tensor memory meanwhile): a task of one or two chunks notices the
     // forty serial initialisations.  Arrival counts: the eight warps of a preparation group or the eight tensor-memory
-    // warps where a whole group signals, four for the L tile (half a group), one everywhere else.
+    // warps where a whole group signals, three for the L tile (its three blocks), one everywhere else.
     constexpr unsigned long long EIGHT = (3ull << B_G_EMPTY) | (3ull << B_P1_FULL) | (3ull << B_O_EMPTY) | (1ull << B_S_READY) |
                                          (7ull << B_QK_EMPTY) | (1ull << B_S_READY_T) | (3ull << B_NORM) | (3ull << B_KDQD_FULL);
     static_assert(PREP_WARPS == 8, "arrival counts of the group barriers");
     for (int i = lane; i < NUM_BARS; i += 32) {
       int count = ((EIGHT >> i) & 1ull) ? 8 : 1;
-      if (i == B_L_FULL || i == B_L_FULL + 1) count = PREP_WARPS / 2;
+      if (i == B_L_FULL || i == B_L_FULL + 1) count = 3;
       // diagnostic switch: the v barriers expect one arrival more than they will ever get, so their waiters give up
       if ((i == B_V_FULL || i == B_V_FULL + 1) && (p.debug_flags & DBG_STALL_V_STREAM)) count = 2;
       mbar_init(x.bar(i), count);
