@@ -304,9 +304,16 @@ def _prepare(q, k, v, g, beta, A_log, dt_bias, scale, initial_state, cu_seqlens,
     lib = _cabi.lib()
     pieces = cut_capacity(T, H) if max_cut_pieces is None else int(max_cut_pieces)
     ws_bytes = lib.kda_prefill_workspace_bytes_cuts(N, H, pieces)
-    workspace = torch.zeros(ws_bytes + 256, dtype=torch.uint8, device=dev)
-    ws_ptr = (workspace.data_ptr() + 255) // 256 * 256
-    status = torch.zeros(4, dtype=torch.int32, device=dev)
+    # One allocation: the four status words, then the workspace.  Cleared is what may be read before a first launch has
+    # written it (the status and, behind the two 48-byte task tables, the counts); the state maps, up to 75 MB, are always
+    # written before they are read.
+    up = lambda b: -(-b // 256) * 256
+    head = 256 + up(48 * (N + 2 * pieces)) + up(48 * N) + 32
+    buf = torch.empty(512 + max(ws_bytes, head), dtype=torch.uint8, device=dev)
+    off = -buf.data_ptr() % 256
+    buf[:off + head].zero_()
+    status = buf[off:off + 16].view(torch.int32)
+    ws_ptr = buf.data_ptr() + off + 256
     out = torch.empty(1, T, H, D, dtype=torch.bfloat16, device=dev)
 
     a = _cabi.KdaPrefillArgs()
@@ -339,7 +346,7 @@ def _prepare(q, k, v, g, beta, A_log, dt_bias, scale, initial_state, cu_seqlens,
     a.kernel = default_kernel() if kernel is None else int(kernel)
     a.max_cut_pieces = pieces
 
-    keep += [q_, k_, v_, g_, beta_, A_, dtb_, cu_seqlens, src, dst, d_idx, s_idx, ck, ck_starts, workspace, status, out]
+    keep += [q_, k_, v_, g_, beta_, A_, dtb_, cu_seqlens, src, dst, d_idx, s_idx, ck, ck_starts, buf, status, out]
     result = (out, dst) if not every else (out, dst, state_checkpoints)
     return _Launch(a, keep, copies, result, status, dev)
 
