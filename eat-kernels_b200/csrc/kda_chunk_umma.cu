@@ -394,10 +394,10 @@ __device__ void role_prep(const ChunkParams& p, const Ctx& x, int grp, int ptid)
         e[2][i] = add2(e[2][i], b1);
         e[3][i] = add2(e[3][i], b1);
       }
-      // The gates are in registers: the tile may be refilled.  Not right behind the loads: an arrival does not wait for loads
-      // in flight (they may sit behind hundreds of cycles of other traffic), only the arithmetic on their values does.
+      // The gates are in registers: the tile may be refilled.  Not right behind the loads, which may sit behind hundreds of
+      // cycles of other traffic: the shuffles behind `own` need every value that a lane has read.
       __syncwarp();
-      if (lane == 0) mbar_arrive(x.bar(B_G_EMPTY + s));
+      if (lane == 0) mbar_arrive_after(x.bar(B_G_EMPTY + s), own[0].x);
       // Range of the primed operands: no exponent exceeds the decay of its half of the chunk.  Beyond 2^126 they are clamped
       // and the intra-chunk products of this chunk are no longer exact: report it.
       const float least = fminf(fminf(fminf(own[0].x, own[0].y), fminf(own[1].x, own[1].y)), fminf(fminf(oth[0].x, oth[0].y), fminf(oth[1].x, oth[1].y)));
@@ -517,7 +517,8 @@ __device__ void role_prep(const ChunkParams& p, const Ctx& x, int grp, int ptid)
         }
       }
       __syncwarp();
-      if (lane == 0) mbar_arrive(x.bar(B_QK_EMPTY + sq));      // the q / k tiles are no longer read
+      // The q / k tiles are no longer read: the last product needs every fragment that the warp has loaded.
+      if (lane == 0) mbar_arrive_after(x.bar(B_QK_EMPTY + sq), acc[0][0]);
       if (rb == cb) {                                          // diagonal block: strictly lower for A, lower for M
         const int m = g + which;
 #pragma unroll

@@ -31,6 +31,14 @@ __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("{\n .reg .b64 st;\n mbarrier.arrive.shared::cta.b64 st, [%0];\n}\n" :: "r"(bar) : "memory");
 }
+// Arrival that hands a tile back to the copy engine, whose next writes are not ordered behind loads that this thread still
+// has in flight: an arrival does not wait for them, and the order of the instructions alone is the compiler's choice.  So it
+// needs `value`, computed from everything that was read (by the whole warp, where an instruction of the whole warp produced
+// it).  The comparison always holds: no arithmetic instruction returns this signalling NaN, the NaN of the hardware is 0x7fffffff.
+__device__ __forceinline__ void mbar_arrive_after(uint32_t bar, float value) {
+  asm volatile("{\n .reg .b64 st;\n .reg .pred p;\n setp.ne.b32 p, %1, 0xff800001;\n @p mbarrier.arrive.shared::cta.b64 st, [%0];\n}\n"
+               :: "r"(bar), "r"(__float_as_uint(value)) : "memory");
+}
 // Potentially blocking test: the hardware may suspend the thread until the phase completes or a time limit of its own
 // passes, so a waiting warp does not take issue slots from the warps it is waiting for.
 __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {

@@ -80,3 +80,30 @@ def test_dt_bias_of_any_alignment(kda, offset):
     res = kda.run(*inputs)
     torch.cuda.synchronize()
     assert all(torch.equal(a, b) for a, b in zip(res, ref))
+
+
+@pytest.mark.parametrize("raw", [True, False])
+def test_a_head_alone_and_among_all(kda, raw):
+    """Every SM busy against a handful of CTAs: a tile handed back to the copy engine before its last read would show as
+    different bits.  Heads are independent, and uncut runs do the same arithmetic in both launches."""
+    H, lens = 48, [1500, 37, 700, 64, 333, 1024]
+    q, k, v, g, beta = plain_on_device(H, sum(lens), 41)
+    init = torch.randn(len(lens), H, D, D, generator=torch.Generator(device=DEV).manual_seed(42), device=DEV) * 0.05
+    if raw:
+        g, beta = g.to(torch.bfloat16), beta.to(torch.bfloat16)
+    A_log, dt_bias = torch.zeros(H, device=DEV), torch.zeros(H * D, device=DEV)
+
+    def call(lo, hi):
+        t = [x[:, :, lo:hi] for x in (q, k, v, g, beta)]
+        s0 = init[:, lo:hi].contiguous()
+        if raw:
+            launch = kda.prepare(*t, A_log[lo:hi], dt_bias[lo * D:hi * D], D ** -0.5, s0, cu_of(lens), max_cut_pieces=0)
+        else:
+            launch = kda.prepare_plain(*t, initial_state=s0, output_final_state=True, cu_seqlens=cu_of(lens), max_cut_pieces=0)
+        return launch()
+
+    out, fin = call(0, H)
+    for h in (0, 17, H - 1):
+        o, f = call(h, h + 1)
+        torch.cuda.synchronize()
+        assert torch.equal(o[:, :, 0], out[:, :, h]) and torch.equal(f[:, 0], fin[:, h])
