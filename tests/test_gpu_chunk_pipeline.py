@@ -107,3 +107,27 @@ def test_a_head_alone_and_among_all(kda, raw):
         o, f = call(h, h + 1)
         torch.cuda.synchronize()
         assert torch.equal(o[:, :, 0], out[:, :, h]) and torch.equal(f[:, 0], fin[:, h])
+
+
+def _rows_before(kda, token, value):
+    """Rows in front of `token`, whose gates are `value` in every channel: the output, the fp64 recurrence, the status."""
+    H, T = 2, 90
+    q, k, v, g, beta = plain_on_device(H, T, 51, 3.0)
+    init = torch.randn(1, H, D, D, generator=torch.Generator(device=DEV).manual_seed(52), device=DEV) * 0.05
+    cut = [t[:, :token].cpu() for t in (q, k, v, g, beta)]
+    g[:, token] = value
+    launch = kda.prepare_plain(q, k, v, g, beta, initial_state=init, output_final_state=True)
+    out, _ = launch()
+    torch.cuda.synchronize()
+    gold, _, _ = gold_plain(*cut, D ** -0.5, init.cpu(), [token])
+    return out[:, :token].float().cpu(), gold, kda.status_bits(launch)
+
+
+@pytest.mark.parametrize("value", [-1e9, float("-inf")])
+@pytest.mark.parametrize("token", [16, 19, 22, 27, 31, 32 + 21, 64 + 25])
+def test_rows_in_front_of_a_reset_keep_their_decay(kda, token, value):
+    """One token of a chunk's second half decays without bound (a state reset): the chunk is reported as out of range, and
+    the tokens in front of that one do not depend on its gates."""
+    out, gold, status = _rows_before(kda, token, value)
+    assert status == 16
+    ko.check_close(out, gold, f"rows in front of token {token}")
