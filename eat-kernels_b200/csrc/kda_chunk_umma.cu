@@ -247,21 +247,38 @@ template <int FE>
 __device__ __forceinline__ float activate_beta(uint32_t raw) { return FE == 1 ? __uint_as_float(raw) : sigmoidf_rel(bf16_lo(raw)); }
 
 // ------------------------------------------------------------------------------------------------ prep warps
-// Step A's exponents, clamped, of a chunk of fp32 gates in which a half decays by more than 2^126.  Where a token decays
-// without bound, taking its token group's sum off the inclusive one has cancelled what precedes the group: here that is added
-// up apart, so that the tokens in front of that one keep their exponents.  Out of line and from the gates in global memory
-// (g: the lane's channels at the first token; the tile may be refilled by now), since in range both forms are as good and any
-// other code in step A is felt: with the same sums beside the others 1 x 8192 at 96 heads took 621 us instead of 609.
-__device__ __noinline__ void wide_exponents(const float* g, long long ld, int lane, int nvalid, float2 (&e)[4][2]) {
+// Step A's exponents, clamped, of a chunk (its first token: t0) in which a half decays by more than 2^126 or a gate is not a
+// number.  Taking the sum of such a gate's token group off the inclusive one has cancelled what precedes the group: here that
+// is added up apart, so that the tokens in front keep their exponents.  Out of line and from the gates in global memory (the
+// tile may be refilled by now), since in range both forms are as good and any other code in step A is felt: with the same
+// sums beside the others 1 x 8192 at 96 heads took 621 us instead of 609.
+template <int FE>
+__device__ __noinline__ void wide_exponents(const ChunkParams& p, long long t0, int nvalid, int h, int ptid, float2 (&e)[4][2]) {
+  const int lane = ptid & 31, ch = 16 * (ptid >> 5) + 4 * (lane & 3);
+  const long long ld = p.ldg, at = t0 * ld + (long long)h * D + ch;
+  const void* g = FE == 1 ? static_cast<const void*>(static_cast<const float*>(p.g) + at) : static_cast<const void*>(static_cast<const __nv_bfloat16*>(p.g) + at);
+  const float* dt_bias = p.dt_bias + h * D + ch;
   const int tg = lane >> 2, sw = ((tg ^ (tg >> 1)) & 1) << 1;
   const bool first = tg < 4, p1 = (tg & 3) >= 1, p2 = (tg & 3) >= 2;
-  const float2 zero = make_float2(0.0f, 0.0f), unit = make_float2(LOG2E, LOG2E);
+  const float2 zero = make_float2(0.0f, 0.0f), unit = FE == 1 ? make_float2(LOG2E, LOG2E) : make_float2(p.lower_bound * LOG2E, p.lower_bound * LOG2E);
+  const float m1 = FE == 0 ? -LOG2E * __expf(p.A_log[h]) : 0.0f;
 #pragma unroll
   for (int j = 0; j < 4; j++) {
     const int tok = (4 * tg + sw) ^ j;
-    const float4 f = tok < nvalid ? *reinterpret_cast<const float4*>(g + tok * ld) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    e[j][0] = make_float2(f.x, f.y);
-    e[j][1] = make_float2(f.z, f.w);
+    e[j][0] = e[j][1] = zero;
+    if (tok >= nvalid) continue;
+    if (FE == 1) {
+      const float4 f = *reinterpret_cast<const float4*>(static_cast<const float*>(g) + tok * ld);
+      e[j][0] = make_float2(f.x, f.y);
+      e[j][1] = make_float2(f.z, f.w);
+    } else {
+      const uint2 f = *reinterpret_cast<const uint2*>(static_cast<const __nv_bfloat16*>(g) + tok * ld);
+#pragma unroll
+      for (int i = 0; i < 2; i++) {
+        const uint32_t w = i ? f.y : f.x;
+        e[j][i] = make_float2(rcpf(1.0f + ex2f(fmaf(bf16_lo(w), m1, m1 * dt_bias[2 * i]))), rcpf(1.0f + ex2f(fmaf(bf16_hi(w), m1, m1 * dt_bias[2 * i + 1]))));
+      }
+    }
   }
 #pragma unroll
   for (int i = 0; i < 2; i++) {
@@ -440,23 +457,16 @@ __device__ void role_prep(const ChunkParams& p, const Ctx& x, int grp, int ptid)
       __syncwarp();
       if (lane == 0) mbar_arrive_after(x.bar(B_G_EMPTY + s), own[0].x);
       // Range of the primed operands: with gates <= 0 no exponent exceeds the decay of its half of the chunk.  Beyond 2^126
-      // they are clamped and the intra-chunk products of this chunk are no longer exact: report it.  (Activated gates are
-      // bounded, so that nothing of them cancels in the sums above.)
-      const float least = fminf(fminf(fminf(own[0].x, own[0].y), fminf(own[1].x, own[1].y)), fminf(fminf(oth[0].x, oth[0].y), fminf(oth[1].x, oth[1].y)));
-      if (__any_sync(0xffffffffu, least < -126.0f)) {
-        if (lane == 0) *range_flag = 1;
-        if (FE == 1) {
-          float2 w[4][2];
-          wide_exponents(static_cast<const float*>(p.g) + (x.t0 + (long long)c * C) * p.ldg + (long long)x.h * D + 16 * pw + 4 * quad, p.ldg, lane, nvalid, w);
+      // they are clamped and the intra-chunk products of this chunk are no longer exact: report it.  (A gate that is not a
+      // number goes the same way, unreported: it shows from its own token on.)
+      const float least = min_nan(min_nan(min_nan(own[0].x, own[0].y), min_nan(own[1].x, own[1].y)), min_nan(min_nan(oth[0].x, oth[0].y), min_nan(oth[1].x, oth[1].y)));
+      if (__any_sync(0xffffffffu, !(least >= -126.0f))) {
+        const float number = fminf(fminf(fminf(own[0].x, own[0].y), fminf(own[1].x, own[1].y)), fminf(fminf(oth[0].x, oth[0].y), fminf(oth[1].x, oth[1].y)));
+        if (number < -126.0f) *range_flag = 1;
+        float2 w[4][2];
+        wide_exponents<FE>(p, x.t0 + (long long)c * C, nvalid, x.h, ptid, w);
 #pragma unroll
-          for (int j = 0; j < 4; j++) { e[j][0] = w[j][0]; e[j][1] = w[j][1]; }
-        } else {
-#pragma unroll
-          for (int j = 0; j < 4; j++)
-#pragma unroll
-            for (int i = 0; i < 2; i++)
-              e[j][i] = first ? make_float2(fminf(e[j][i].x, 126.0f), fminf(e[j][i].y, 126.0f)) : make_float2(fmaxf(e[j][i].x, -126.0f), fmaxf(e[j][i].y, -126.0f));
-        }
+        for (int j = 0; j < 4; j++) { e[j][0] = w[j][0]; e[j][1] = w[j][1]; }
       }
 #pragma unroll
       for (int i = 0; i < 2; i++) {
@@ -1213,7 +1223,7 @@ __device__ void role_tmem_dual(const ChunkParams& p, const Task& task, const Ctx
 
 // ------------------------------------------------------------------------------------------------ kernel
 template <int FE, int KF>
-__global__ void __launch_bounds__(THREADS, 1) kda_chunk_umma_kernel(const ChunkParams p, const __grid_constant__ TmaMaps maps) {
+__global__ void __launch_bounds__(THREADS, 1) kda_chunk_umma_kernel(const __grid_constant__ ChunkParams p, const __grid_constant__ TmaMaps maps) {
   extern __shared__ __align__(1024) uint8_t smem[];
   const int tid = threadIdx.x, lane = tid & 31;
   const int warp = tid >> 5;

@@ -131,3 +131,21 @@ def test_rows_in_front_of_a_reset_keep_their_decay(kda, token, value):
     out, gold, status = _rows_before(kda, token, value)
     assert status == 16
     ko.check_close(out, gold, f"rows in front of token {token}")
+
+
+@pytest.mark.parametrize("token", [16, 19, 27, 31, 32 + 21, 64 + 25])
+def test_rows_in_front_of_a_gate_that_is_not_a_number(kda, token):
+    """A NaN gate in a chunk's second half reaches its own token and what follows, not the rows in front of it."""
+    out, gold, status = _rows_before(kda, token, float("nan"))
+    assert status == 0
+    ko.check_close(out, gold, f"rows in front of token {token}")
+
+
+@pytest.mark.parametrize("token", [16, 19, 27, 31, 32 + 21, 64 + 25])
+def test_rows_in_front_of_a_raw_gate_that_is_not_a_number(kda, token):
+    inputs = ko.make_inputs_raw(2, [90], 53)
+    gold, _, _ = gold_raw([t[:, :token] for t in inputs[:5]] + list(inputs[5:9]), [token])
+    inputs[3][:, token] = float("nan")
+    out, _ = kda.run(*to_dev(inputs))
+    torch.cuda.synchronize()
+    ko.check_close(out[:, :token].float().cpu(), gold, f"rows in front of token {token}")
