@@ -24,10 +24,12 @@ unsigned long long* g_prof = nullptr;
 inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
+constexpr size_t kCountBytes = 256;    // the counts lie at the front: a caller clears them without knowing the rest
+
 struct Workspace {
+  int* n_tasks;            // [0] first launch, [1] second launch, [2] scan chains
   kda::Task* tasks;
   kda::Task* tasks_unsorted;
-  int* n_tasks;            // [0] first launch, [1] second launch, [2] scan chains
   long long* cu_safe;
   float* trash;
   // only with cuts (max_pieces > 0)
@@ -45,9 +47,9 @@ Workspace carve(void* base, int N, int H, int pieces = 0) {
   uint8_t* b = reinterpret_cast<uint8_t*>(base);
   const size_t n = (size_t)(N > 0 ? N : 1);
   const size_t na = n + 2 * (size_t)pieces;
+  w.n_tasks = reinterpret_cast<int*>(b + off); off += kCountBytes;
   w.tasks = reinterpret_cast<kda::Task*>(b + off); off = align_up(off + na * sizeof(kda::Task), 256);
   w.tasks_unsorted = reinterpret_cast<kda::Task*>(b + off); off = align_up(off + n * sizeof(kda::Task), 256);
-  w.n_tasks = reinterpret_cast<int*>(b + off); off = align_up(off + 32, 256);
   w.cu_safe = reinterpret_cast<long long*>(b + off); off = align_up(off + (n + 1) * sizeof(long long), 256);
   w.trash = reinterpret_cast<float*>(b + off); off = align_up(off + (size_t)H * kda::STATE_ELEMS * sizeof(float), 256);
   w.tasks_b = nullptr; w.chains = nullptr; w.map_P = w.map_L = w.map_E = nullptr;
@@ -173,6 +175,8 @@ size_t kda_prefill_workspace_bytes_cuts(int32_t N, int32_t H, int32_t max_cut_pi
   if (N < 0 || H <= 0 || max_cut_pieces < 0 || max_cut_pieces > KDA_MAX_CUT_PIECES) return 0;
   return carve(nullptr, N, H, max_cut_pieces).bytes;
 }
+
+size_t kda_prefill_workspace_clear_bytes(void) { return kCountBytes; }
 
 int kda_prefill_launch(const KdaPrefillArgs* a, void* stream_) {
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);

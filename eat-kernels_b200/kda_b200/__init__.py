@@ -305,13 +305,11 @@ def _prepare(q, k, v, g, beta, A_log, dt_bias, scale, initial_state, cu_seqlens,
     pieces = cut_capacity(T, H) if max_cut_pieces is None else int(max_cut_pieces)
     ws_bytes = lib.kda_prefill_workspace_bytes_cuts(N, H, pieces)
     # One allocation: the four status words, then the workspace.  Cleared is what may be read before a first launch has
-    # written it (the status and, behind the two 48-byte task tables, the counts); the state maps, up to 75 MB, are always
-    # written before they are read.
-    up = lambda b: -(-b // 256) * 256
-    head = 256 + up(48 * (N + 2 * pieces)) + up(48 * N) + 32
-    buf = torch.empty(512 + max(ws_bytes, head), dtype=torch.uint8, device=dev)
+    # written it (the status and the counts at the workspace's front); the state maps, up to 75 MB, are always written
+    # before they are read.
+    buf = torch.empty(512 + ws_bytes, dtype=torch.uint8, device=dev)
     off = -buf.data_ptr() % 256
-    buf[:off + head].zero_()
+    buf[:off + 256 + lib.kda_prefill_workspace_clear_bytes()].zero_()
     status = buf[off:off + 16].view(torch.int32)
     ws_ptr = buf.data_ptr() + off + 256
     out = torch.empty(1, T, H, D, dtype=torch.bfloat16, device=dev)

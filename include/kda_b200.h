@@ -140,6 +140,9 @@ typedef struct KdaPrefillArgs {
 size_t kda_prefill_workspace_bytes(int32_t N, int32_t H);
 /* The same with room for the state maps of `max_cut_pieces` pieces (3 x 64 KB per piece and head). */
 size_t kda_prefill_workspace_bytes_cuts(int32_t N, int32_t H, int32_t max_cut_pieces);
+/* Bytes at the front of a workspace to clear if kda_prefill_plan_counts may be asked before the first launch has run.  A
+ * launch needs nothing cleared: it writes what it reads. */
+size_t kda_prefill_workspace_clear_bytes(void);
 
 /* Validates the caller's tables on the device, orders the (sequence, head) tasks longest first and runs the fused
  * chunk kernel.  Two kernel launches (four with max_cut_pieces >= 2: planner, chunk kernel, scan of the cut sequences'
