@@ -148,14 +148,26 @@ class _Launch:
     """Zero-argument launch closure.  Owns the output, workspace and status tensors; every call re-reads the caller's
     buffers (same addresses) and enqueues two kernels on the current stream."""
 
-    def __init__(self, args, keep, copies, result, status, device):
+    def __init__(self, args, keep, copies, result, scratch, device):
         self._args = args
         self._keep = keep          # tensors whose storage the argument block points into
         self._copies = copies      # (private contiguous copy, caller tensor) pairs refreshed at every call
         self._result = result
-        self.status = status
+        self._scratch = scratch    # the status words and, 256 bytes behind them, the workspace
         self._device = device
         self._lib = _cabi.lib()
+
+    @property
+    def status(self):
+        at = self._args.status - self._scratch.data_ptr()
+        return self._scratch[at:at + 16].view(torch.int32)
+
+    def _cleared(self):
+        """What may be asked for before a first launch has written it, the status and the planner's counts, set to zero.  The
+        launch itself needs nothing cleared, so a call that launches at once saves the fill."""
+        end = self._args.workspace + self._lib.kda_prefill_workspace_clear_bytes() - self._scratch.data_ptr()
+        self._scratch[:end].zero_()
+        return self
 
     def __call__(self):
         for c, t in self._copies:
@@ -304,14 +316,8 @@ def _prepare(q, k, v, g, beta, A_log, dt_bias, scale, initial_state, cu_seqlens,
     lib = _cabi.lib()
     pieces = cut_capacity(T, H) if max_cut_pieces is None else int(max_cut_pieces)
     ws_bytes = lib.kda_prefill_workspace_bytes_cuts(N, H, pieces)
-    # One allocation: the four status words, then the workspace.  Cleared is what may be read before a first launch has
-    # written it (the status and the counts at the workspace's front); the state maps, up to 75 MB, are always written
-    # before they are read.
-    buf = torch.empty(512 + ws_bytes, dtype=torch.uint8, device=dev)
-    off = -buf.data_ptr() % 256
-    buf[:off + 256 + lib.kda_prefill_workspace_clear_bytes()].zero_()
-    status = buf[off:off + 16].view(torch.int32)
-    ws_ptr = buf.data_ptr() + off + 256
+    scratch = torch.empty(512 + ws_bytes, dtype=torch.uint8, device=dev)       # the status words, then the workspace
+    status_ptr = (scratch.data_ptr() + 255) // 256 * 256
     out = torch.empty(1, T, H, D, dtype=torch.bfloat16, device=dev)
 
     a = _cabi.KdaPrefillArgs()
@@ -339,14 +345,21 @@ def _prepare(q, k, v, g, beta, A_log, dt_bias, scale, initial_state, cu_seqlens,
     if every:
         a.ck_base, a.ck_is_bf16, a.ck_every, a.ck_rows = ck.data_ptr(), int(ck.dtype == torch.bfloat16), every, ck.shape[0]
         a.ck_starts, a.ck_starts_is64 = ck_starts.data_ptr(), int(ck_starts.dtype == torch.int64)
-    a.workspace, a.workspace_bytes = ws_ptr, ws_bytes
-    a.status = status.data_ptr()
+    a.workspace, a.workspace_bytes = status_ptr + 256, ws_bytes
+    a.status = status_ptr
     a.kernel = default_kernel() if kernel is None else int(kernel)
     a.max_cut_pieces = pieces
 
-    keep += [q_, k_, v_, g_, beta_, A_, dtb_, cu_seqlens, src, dst, d_idx, s_idx, ck, ck_starts, buf, status, out]
+    keep += [q_, k_, v_, g_, beta_, A_, dtb_, cu_seqlens, src, dst, d_idx, s_idx, ck, ck_starts, scratch, out]
     result = (out, dst) if not every else (out, dst, state_checkpoints)
-    return _Launch(a, keep, copies, result, status, dev)
+    return _Launch(a, keep, copies, result, scratch, dev)
+
+
+def _prepare_raw(q, k, v, g, beta, A_log, dt_bias, scale, initial_state, cu_seqlens, dynamic_layout, serving):
+    if initial_state is None and serving.get("initial_state_source") is None:
+        raise _err("initial_state is required unless only initial_state_source is given")
+    return _prepare(q, k, v, g, beta, A_log, dt_bias, scale, initial_state, cu_seqlens, raw=True, key_first=False,
+                    dynamic_layout=dynamic_layout, **serving)
 
 
 def prepare(q, k, v, g, beta, A_log, dt_bias, scale, initial_state, cu_seqlens=None, *, dynamic_layout=False, **serving):
@@ -354,15 +367,12 @@ def prepare(q, k, v, g, beta, A_log, dt_bias, scale, initial_state, cu_seqlens=N
     every input buffer.  The schedule is always derived on the device from cu_seqlens, so both settings are CUDA-graph
     safe; `dynamic_layout=True` additionally insists that the tables are contiguous device tensors read in place
     (kda/b200/kda_b200.py:49-53).  Without a pool, `initial_state` is read-only and the final state is a new tensor."""
-    if initial_state is None and serving.get("initial_state_source") is None:
-        raise _err("initial_state is required unless only initial_state_source is given")
-    return _prepare(q, k, v, g, beta, A_log, dt_bias, scale, initial_state, cu_seqlens, raw=True, key_first=False,
-                    dynamic_layout=dynamic_layout, **serving)
+    return _prepare_raw(q, k, v, g, beta, A_log, dt_bias, scale, initial_state, cu_seqlens, dynamic_layout, serving)._cleared()
 
 
 def run(q, k, v, g, beta, A_log, dt_bias, scale, initial_state, cu_seqlens=None, **serving):
     """run(...) -> (output, final_state[, state_checkpoints]); the serving entry point (kda/b200/kda_b200.py:44-47)."""
-    return prepare(q, k, v, g, beta, A_log, dt_bias, scale, initial_state, cu_seqlens, dynamic_layout=True, **serving)()
+    return _prepare_raw(q, k, v, g, beta, A_log, dt_bias, scale, initial_state, cu_seqlens, True, serving)()
 
 
 def kda_prefill(q, k, v, g, beta, A_log, dt_bias, initial_state, cu_seqlens=None, scale=None, *,
@@ -377,8 +387,7 @@ def kda_prefill(q, k, v, g, beta, A_log, dt_bias, initial_state, cu_seqlens=None
                initial_state_source=initial_state_source, initial_state_indices=initial_state_indices)
 
 
-def prepare_plain(q, k, v, g, beta, scale=None, initial_state=None, output_final_state=False, cu_seqlens=None, **serving):
-    """Launch closure of the pre-activated call (see chunk_kda)."""
+def _prepare_plain(q, k, v, g, beta, scale, initial_state, output_final_state, cu_seqlens, serving):
     if q.dim() == 4 and q.shape[0] > 1:
         if cu_seqlens is not None:
             raise _err("cu_seqlens needs batch size 1 (packed varlen layout)")
@@ -392,11 +401,16 @@ def prepare_plain(q, k, v, g, beta, scale=None, initial_state=None, output_final
                     want_final=output_final_state or "ssm_state_indices" in serving, **serving)
 
 
+def prepare_plain(q, k, v, g, beta, scale=None, initial_state=None, output_final_state=False, cu_seqlens=None, **serving):
+    """Launch closure of the pre-activated call (see chunk_kda)."""
+    return _prepare_plain(q, k, v, g, beta, scale, initial_state, output_final_state, cu_seqlens, serving)._cleared()
+
+
 def chunk_kda(q, k, v, g, beta, scale=None, initial_state=None, output_final_state=False, cu_seqlens=None, **serving):
     """Plain `chunk_kda`-style call with PRE-ACTIVATED inputs: q, k already L2-normalised, g the fp32 log-decay (<= 0)
     per token / head / key channel, beta fp32 in (0, 1); state key-first [N, H, K, V] fp32.  q, k, v are read as bf16
     (other dtypes are cast).  Returns (o [B, T, H, 128] in q's dtype, final_state or None)."""
     shape, dt = q.shape, q.dtype
-    res = prepare_plain(q, k, v, g, beta, scale, initial_state, output_final_state, cu_seqlens, **serving)()
+    res = _prepare_plain(q, k, v, g, beta, scale, initial_state, output_final_state, cu_seqlens, serving)()
     o = res[0].reshape(shape)
     return (o if dt == torch.bfloat16 else o.to(dt), *res[1:])

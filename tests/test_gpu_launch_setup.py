@@ -5,7 +5,7 @@ import pytest
 import torch
 
 import kda_oracle as ko
-from kda_testlib import DEV, cu_of, plain_on_device, to_dev
+from kda_testlib import DEV, plain_on_device, to_dev
 
 pytestmark = pytest.mark.gpu
 
@@ -50,3 +50,31 @@ def test_nothing_is_reported_before_the_first_launch(kda, heads, lens):
         launch()
         torch.cuda.synchronize()
         assert launch.plan_counts()[0] >= len(lens) and kda.status_bits(launch) == 0
+
+
+@pytest.mark.parametrize("raw", [True, False])
+def test_a_call_that_launches_at_once_fills_nothing(kda, raw):
+    """The planner writes the status and the counts of every launch before anything reads them, so the one-shot calls enqueue
+    the library's kernels and nothing in front of them."""
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    class Ops(TorchDispatchMode):
+        def __init__(self):
+            super().__init__()
+            self.names = []
+
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            self.names.append(str(func))
+            return func(*args, **(kwargs or {}))
+
+    H, lens = 4, [300, 77]
+    inputs = to_dev(ko.make_inputs_raw(H, lens, 62))
+    plain = plain_on_device(H, sum(lens), 63)
+    with Ops() as ops:
+        if raw:
+            res = kda.run(*inputs)
+        else:
+            res = kda.chunk_kda(*plain, output_final_state=True, cu_seqlens=inputs[9])
+    torch.cuda.synchronize()
+    assert res[0].shape == (1, sum(lens), H, 128)
+    assert not [n for n in ops.names if any(w in n for w in ("zero", "fill", "copy", "ones", "full"))], ops.names
