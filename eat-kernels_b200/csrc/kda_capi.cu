@@ -316,13 +316,15 @@ int kda_segment_launch(const KdaSegmentArgs* s, void* stream_) {
     if (!aligned16(s->tiles) || s->n_tiles < 0) return KDA_ERR_ARG;
     sp.tiles = reinterpret_cast<__nv_bfloat16*>(s->tiles);
   }
+  // Qt rows (with tiles nothing is written there): any whole value on the tcgen05 kernel, 16-byte stores on the other one
+  if (!sp.dual && (reinterpret_cast<uintptr_t>(s->qt) & (a->kernel == KDA_KERNEL_MMA_SYNC ? 15 : 1)) != 0) return KDA_ERR_ARG;
   sp.P = s->P; sp.S_loc = s->S_loc;
   sp.tasks = w.tasks; sp.n_tasks = w.n_tasks; sp.status = a->status;
   cudaError_t e = kda::launch_seg_plan(sp, stream);
   if (e != cudaSuccess) return cuda_fail(e);
   kda::ChunkParams p;
   fill_chunk_params(p, a);
-  p.out_aux = reinterpret_cast<__nv_bfloat16*>(s->qt);
+  p.out_aux = sp.dual ? nullptr : reinterpret_cast<__nv_bfloat16*>(s->qt);
   p.oloc_tile_offset = s->n_tiles * a->H * (long long)(KDA_HEAD_DIM * KDA_CHUNK);
   p.key_first = 0;
   p.tasks = w.tasks;

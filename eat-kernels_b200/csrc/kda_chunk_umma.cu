@@ -924,13 +924,24 @@ __device__ __forceinline__ void decay64(uint32_t tS, const float* dcol, int lane
   tmem_wait_st();
 }
 
+// two neighbouring bf16 values of an output row
+template <int PAIRS>
+__device__ __forceinline__ void store_pair(__nv_bfloat16* at, uint32_t w) {
+  if (PAIRS) {
+    *reinterpret_cast<uint32_t*>(at) = w;
+  } else {
+    reinterpret_cast<uint16_t*>(at)[0] = (uint16_t)w;
+    reinterpret_cast<uint16_t*>(at)[1] = (uint16_t)(w >> 16);
+  }
+}
+
 // Eight warps own the tensor-memory traffic that goes through registers: warp (quarter q, half hf) serves the 32
 // value rows [32 q, 32 q + 32) (the tensor-memory lanes a warp with id % 4 == q may touch) and, of those, the state
 // columns [64 hf, 64 hf + 64) and the output tokens [16 hf, 16 hf + 16) of every chunk.  Per chunk:
 //   wait MMA1 done -> (checkpoint row if due) -> St <- St diag(2^G31) for its columns -> signal S_READY        (on the chain)
 //   wait MMA3 done -> O columns -> registers -> release the O buffer -> bf16 -> global                         (off the chain)
 // plus the initial state load and the final state store for its columns.
-template <int KF>
+template <int KF, int PAIRS>
 __device__ void role_tmem(const ChunkParams& p, const Task& task, const Ctx& x, uint32_t tmem, int quarter, int hf, int lane) {
   const int v = 32 * quarter + lane;
   const uint32_t lane_base = (uint32_t)(32 * quarter) << 16;
@@ -966,7 +977,7 @@ __device__ void role_tmem(const ChunkParams& p, const Task& task, const Ctx& x, 
   if (lane == 0) mbar_arrive(x.bar(B_S_READY));
 
   // Output: the two lanes of a pair exchange halves, so that a lane stores two neighbouring values of one token (even lanes
-  // the even tokens) instead of one value of every token.
+  // the even tokens) instead of one value of every token.  Rows that are not aligned to that (PAIRS = 0) are stored by value.
   const bool odd = lane & 1;
   const bool write_out = !(task.flags & TF_NO_OUT);
   const long long ldo = p.ldo;
@@ -1021,11 +1032,11 @@ __device__ void role_tmem(const ChunkParams& p, const Task& task, const Ctx& x, 
       const int left = x.len - c * C - 16 * hf - (int)odd;     // tokens of this run from this lane's first one on
       if (x.len - c * C >= C) {
 #pragma unroll
-        for (int i = 0; i < 8; i++) *reinterpret_cast<uint32_t*>(orow + (long long)(2 * i) * ldo) = w[i];
+        for (int i = 0; i < 8; i++) store_pair<PAIRS>(orow + (long long)(2 * i) * ldo, w[i]);
       } else {
 #pragma unroll
         for (int i = 0; i < 8; i++)
-          if (2 * i < left) *reinterpret_cast<uint32_t*>(orow + (long long)(2 * i) * ldo) = w[i];
+          if (2 * i < left) store_pair<PAIRS>(orow + (long long)(2 * i) * ldo, w[i]);
       }
     }
   }
@@ -1222,7 +1233,7 @@ __device__ void role_tmem_dual(const ChunkParams& p, const Task& task, const Ctx
 }
 
 // ------------------------------------------------------------------------------------------------ kernel
-template <int FE, int KF>
+template <int FE, int KF, int PAIRS>
 __global__ void __launch_bounds__(THREADS, 1) kda_chunk_umma_kernel(const __grid_constant__ ChunkParams p, const __grid_constant__ TmaMaps maps) {
   extern __shared__ __align__(1024) uint8_t smem[];
   const int tid = threadIdx.x, lane = tid & 31;
@@ -1322,7 +1333,7 @@ __global__ void __launch_bounds__(THREADS, 1) kda_chunk_umma_kernel(const __grid
     __syncwarp();
   } else if (warp < W_PREP0) {
     if (dual) role_tmem_dual<KF>(p, task, x, tmem, warp & 3, (warp - W_SCALE0) >> 2, lane);
-    else role_tmem<KF>(p, task, x, tmem, warp & 3, (warp - W_SCALE0) >> 2, lane);
+    else role_tmem<KF, PAIRS>(p, task, x, tmem, warp & 3, (warp - W_SCALE0) >> 2, lane);
   } else {
     const int pt = tid - W_PREP0 * 32;
     role_prep<FE>(p, x, pt / PREP_THREADS, pt % PREP_THREADS);
@@ -1347,16 +1358,17 @@ __global__ void __launch_bounds__(THREADS, 1) kda_chunk_umma_kernel(const __grid
 }  // namespace u
 
 cudaError_t launch_chunk_umma(const ChunkParams& p, const TmaMaps& maps, int n_task_cap, cudaStream_t stream, bool after_planner) {
-  // one instantiation per (front-end, state layout): smaller code per launch, and instruction-cache footprint is what
-  // bounds this role-specialised kernel
+  // One instantiation per (front-end, state layout).  Those of the third row are for Qt rows at an address that is no multiple
+  // of four (value-first only, as every segment launch): a test of it per chunk cost the others up to 4 %.
   typedef void (*Kern)(const ChunkParams, const TmaMaps);
-  static const Kern kerns[2][2] = {{u::kda_chunk_umma_kernel<0, 0>, u::kda_chunk_umma_kernel<0, 1>},
-                                   {u::kda_chunk_umma_kernel<1, 0>, u::kda_chunk_umma_kernel<1, 1>}};
+  static const Kern kerns[3][2] = {{u::kda_chunk_umma_kernel<0, 0, 1>, u::kda_chunk_umma_kernel<0, 1, 1>},
+                                   {u::kda_chunk_umma_kernel<1, 0, 1>, u::kda_chunk_umma_kernel<1, 1, 1>},
+                                   {u::kda_chunk_umma_kernel<0, 0, 0>, u::kda_chunk_umma_kernel<1, 0, 0>}};
   static int attr_dev_mask = 0;
   int dev = 0;
   cudaGetDevice(&dev);
   if (!(attr_dev_mask & (1 << (dev & 31)))) {
-    for (int i = 0; i < 4; i++) {
+    for (int i = 0; i < 6; i++) {
       cudaError_t e = cudaFuncSetAttribute(kerns[i >> 1][i & 1], cudaFuncAttributeMaxDynamicSharedMemorySize, u::SMEM_BYTES);
       if (e != cudaSuccess) return e;
     }
@@ -1376,7 +1388,9 @@ cudaError_t launch_chunk_umma(const ChunkParams& p, const TmaMaps& maps, int n_t
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = after_planner ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, kerns[p.frontend ? 1 : 0][p.key_first ? 1 : 0], p, maps);
+  const bool unpaired = (reinterpret_cast<uintptr_t>(p.out_aux) & 3) != 0;
+  if (unpaired && p.key_first) return cudaErrorInvalidValue;
+  return cudaLaunchKernelEx(&cfg, unpaired ? kerns[2][p.frontend ? 1 : 0] : kerns[p.frontend ? 1 : 0][p.key_first ? 1 : 0], p, maps);
 }
 
 }  // namespace kda

@@ -55,6 +55,19 @@ def test_null_arguments_are_rejected_without_a_device(lib):
     assert lib.kda_fixup_tiles_launch(None, None, 0, 0, None, None, None, None, 1, 1, 0, None) == -1
 
 
+@pytest.mark.parametrize("kernel,qt", [(1, 0x10008), (1, 0x10002), (0, 0x10001), (2, 0x10001), (2, 0x10003)])
+def test_qt_rows_that_a_kernel_cannot_store_to_are_rejected_without_a_device(lib, kernel, qt):
+    from kda_b200 import _cabi
+    s = _cabi.KdaSegmentArgs()
+    a = s.base
+    a.q = a.k = a.v = a.g = a.beta = a.out = a.status = a.workspace = a.A_log = a.dt_bias = 0x10000
+    a.ldq = a.ldk = a.ldv = a.ldg = a.ldo = 128
+    a.ldbeta = a.H = a.N = 1
+    a.T, a.kernel, a.workspace_bytes = 32, kernel, lib.kda_prefill_workspace_bytes(2, 1)
+    s.n_seg, s.seg_t0, s.seg_t1, s.seg_need_map, s.P, s.S_loc, s.qt = 1, 0x10000, 0x10000, 0x10000, 0x10000, 0x10000, qt
+    assert lib.kda_segment_launch(ctypes.byref(s), None) == -1
+
+
 def test_segment_tiles_counts_tiles_of_32_tokens_per_segment(lib):
     """Host helper that sizes the tile-major scratch of a segment launch: every segment rounds up on its own, tables
     are clamped to [0, T] as the device planner clamps them."""

@@ -228,3 +228,32 @@ def test_cut_sequence_matches_the_serving_call(kda, H, T, every, pieces, ck_dtyp
     if every:
         ko.check_close(res["cut"][2][row0:row0 + rows].float().cpu(), res["plain"][2][row0:row0 + rows].float().cpu(), tag + " checkpoint rows")
         assert torch.isnan(res["cut"][2][:row0].float()).all() and torch.isnan(res["cut"][2][row0 + rows:].float()).all(), tag + ": rows outside the range written"
+
+
+def test_qt_rows_may_lie_at_any_even_address(kda):
+    """The two-task scheme writes Qt as rows; an address that is no multiple of four bytes gives the same rows."""
+    from kda_b200 import parallel
+    H, bounds = 3, [0, 33, 97, 300]
+    T = bounds[-1]
+    q, k, v, g, beta, A_log, dt_bias, scale, _, _ = to_dev(ko.make_inputs_raw(H, [T], 95))
+
+    class Backend(parallel.CudaBackend):
+        shift = 0
+
+        def _buf(self, key, shape, dtype, dev, zero=False):
+            if key != "qt":
+                return super()._buf(key, shape, dtype, dev, zero)
+            n = T * H * D
+            return torch.full((n + 8,), float("nan"), dtype=dtype, device=dev)[self.shift:self.shift + n].view(shape)
+
+    res = []
+    for shift in (0, 1, 2):
+        be = Backend(dual=False)
+        be.shift = shift
+        out, qt, P, S_loc = be.segment_maps(q, k, v, g, beta, A_log, dt_bias, scale, True, bounds, [1, 1, 1], None)
+        assert qt.data_ptr() % 4 == (2 * shift) % 4
+        torch.cuda.synchronize()
+        assert be.kernel_error() == 0
+        res.append([t.clone() for t in (out, qt, P, S_loc)])
+    for other in res[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(res[0], other))
