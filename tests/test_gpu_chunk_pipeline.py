@@ -149,3 +149,35 @@ def test_rows_in_front_of_a_raw_gate_that_is_not_a_number(kda, token):
     out, _ = kda.run(*to_dev(inputs))
     torch.cuda.synchronize()
     ko.check_close(out[:, :token].float().cpu(), gold, f"rows in front of token {token}")
+
+
+@pytest.mark.parametrize("raw", [True, False])
+def test_strided_tokens_of_the_least_alignment(kda, raw):
+    """q, k, v, g as slices whose base and token stride are multiples of 16 bytes and of nothing more: read in place."""
+    H, lens = 3, [70, 1, 161]
+    T = sum(lens)
+    q, k, v, g, beta = plain_on_device(H, T, 71)
+    if raw:
+        g, beta = g.to(torch.bfloat16), beta.to(torch.bfloat16)
+    A_log, dt_bias = torch.zeros(H, device=DEV), torch.zeros(H * D, device=DEV)
+    init = torch.randn(len(lens), H, D, D, generator=torch.Generator(device=DEV).manual_seed(72), device=DEV) * 0.05
+
+    def sliced(t):
+        pad = 16 // t.element_size() if t.element_size() == 2 else 8     # (the token stride: a multiple of eight elements)
+        wide = torch.full((T, H * D + 3 * pad), float("nan"), dtype=t.dtype, device=DEV)
+        part = wide[:, 16 // t.element_size():][:, :H * D]
+        part.copy_(t.view(T, H * D))
+        return part.unflatten(1, (H, D))[None]
+
+    def launch(t):
+        if raw:
+            return kda.prepare(*t, beta, A_log, dt_bias, D ** -0.5, init, cu_of(lens))
+        return kda.prepare_plain(*t, beta, initial_state=init, output_final_state=True, cu_seqlens=cu_of(lens))
+
+    views = [sliced(t) for t in (q, k, v, g)]
+    assert all(t.data_ptr() % 32 == 16 for t in views)
+    there, here = launch(views), launch([q, k, v, g])
+    assert there._copies == []
+    a, b = there(), here()
+    torch.cuda.synchronize()
+    assert all(torch.equal(x, y) for x, y in zip(a, b))
