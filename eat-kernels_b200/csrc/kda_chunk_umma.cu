@@ -77,7 +77,7 @@ constexpr int OFF_L = OFF_TBH + 4096;                         // 2 x fp32 [32][L
 constexpr int OFF_DEC = OFF_L + 2 * C * LS * 4;               // 4 x 512 (a slot is rewritten four chunks later)
 constexpr int OFF_BETA = OFF_DEC + 2048;                      // beta of a chunk: 2 groups x 2 (alternating) x 128
 constexpr int OFF_BAR = OFF_BETA + 512;                       // mbarriers
-constexpr int NUM_BARS = 43;
+constexpr int NUM_BARS = 42;
 constexpr int OFF_MISC = OFF_BAR + NUM_BARS * 8;              // +0 tmem slot, +8 abort code, +12 range flag, +16 wait limit (ns)
 constexpr int SMEM_BYTES = OFF_MISC + 64;
 static_assert(SMEM_BYTES <= 227 * 1024 && STAGE % 1024 == 0 && OFF_MISC % 8 == 0, "shared memory budget");
@@ -327,7 +327,10 @@ __device__ void role_prep(const ChunkParams& p, const Ctx& x, int grp, int ptid)
   float* norm = reinterpret_cast<float*>(x.smem + OFF_NORM) + s * 128;
   int sq = grp, fq = grp;                              // q / k stage of the chunk, its full barrier and parity
   uint32_t pq = 0;
-  // offsets of step 0 (step j: ^ j * 0x90 for rows of 128 bytes, ^ j * 0xa0 for kr)
+  // offsets of step 0 (step j: ^ j * 0x90 for rows of 128 bytes, ^ j * 0xa0 for kr).  kr is MN-major in the 128-byte swizzle
+  // with 32-byte base: token rows of 32 channels, 32-byte pieces XOR-ed with (token % 4), four rows to a 512-byte atom,
+  // atoms 512 bytes apart along the channels and 2048 along the tokens.  (Written out: through a helper with the general
+  // form the raw-gate instantiations spill 16 bytes more and 1 x 32768 with checkpoints takes 5 % longer.)
   const uint32_t off_f32 = (uint32_t)(tok0 * 128 + (((4 * (pw & 1) + quad) ^ (tok0 & 7)) << 4));
   const uint32_t off_g = FE == 1 ? (uint32_t)((pw >> 1) * 4096) + off_f32 : 0u;
   const uint32_t off_kd = (uint32_t)((pw >> 1) * 8192) + off_f32;

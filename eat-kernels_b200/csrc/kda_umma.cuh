@@ -8,8 +8,8 @@
 //                       advancing the descriptor's start address inside the 128-byte row.
 //       MN-major SW128: rows are K indices holding 128 bytes of M/N-contiguous data, 8 K-rows form a 1024-byte atom;
 //                       LBO = byte distance between atoms along M/N, SBO = byte distance between 8-row K groups.
-//                       (16-bit operands; 32-bit MN-major operands need the 32-byte-base variant, see
-//                       mnmajor_f32_off.)
+//                       (16-bit operands.  32-bit MN-major operands need the variant with 32-byte base, layout type 1:
+//                       4 K-rows form a 512-byte atom whose 32-byte pieces are XOR-swizzled with (K % 4).)
 //     Tiles are 1024-byte aligned so that the address-bit swizzle of the hardware equals the (row % 8) rule above.
 //   * Every wait on an mbarrier is bounded: after `limit_ns` of wall time (kWaitLimitNs unless the launch overrides it)
 //     the waiter raises the CTA's abort flag and carries on as if the wait had succeeded, so control flow (and every
@@ -227,18 +227,6 @@ __device__ __forceinline__ void mma_commit_pred(uint32_t bar, uint32_t go) {
 __device__ __forceinline__ uint32_t kmajor_f32_off(int row, int k, uint32_t kblock_bytes) {
   return (uint32_t)(k >> 5) * kblock_bytes + (uint32_t)(row >> 3) * 1024u + (uint32_t)(row & 7) * 128u +
          (uint32_t)((((k & 31) >> 2) ^ (row & 7)) << 4) + (uint32_t)(k & 3) * 4u;
-}
-// MN-major tile of 32-bit elements in the 128-byte swizzle with 32-byte base (layout type 1, the only MN-major form
-// the tensor core accepts for tf32): K rows of 128 bytes (32 M/N elements), 4 K-rows form a 512-byte atom whose
-// 32-byte pieces are XOR-ed with (k % 4); atom (mn block, k group of 4) at mn_block * lbo + k_group * sbo.
-__device__ __forceinline__ uint32_t mnmajor_f32_off(int mn, int k, uint32_t lbo, uint32_t sbo) {
-  return (uint32_t)(mn >> 5) * lbo + (uint32_t)(k >> 2) * sbo + (uint32_t)(k & 3) * 128u +
-         (uint32_t)((((mn & 31) >> 3) ^ (k & 3)) << 5) + (uint32_t)(mn & 7) * 4u;
-}
-// MN-major SW128 tile of 16-bit elements (64 M/N elements per 128-byte row).
-__device__ __forceinline__ uint32_t mnmajor_b16_off(int mn, int k, uint32_t lbo, uint32_t sbo) {
-  return (uint32_t)(mn >> 6) * lbo + (uint32_t)(k >> 3) * sbo + (uint32_t)(k & 7) * 128u +
-         (uint32_t)((((mn & 63) >> 3) ^ (k & 7)) << 4) + (uint32_t)(mn & 7) * 2u;
 }
 // K-major SW64 tile of 16-bit elements: rows of 64 bytes (32 elements), 8-row groups 512 B apart; the 16-byte chunk
 // index is XOR-ed with address bits [7,9) = (row / 2) % 4.
