@@ -120,7 +120,8 @@ void fill_chunk_params(kda::ChunkParams& p, const KdaPrefillArgs* a) {
   p.prof = g_prof;
 }
 
-// Tensor maps of the token tensors for the tcgen05 kernel's copy engine (see kda_tma.cuh).  T == 0: nothing is ever copied, the maps stay zeroed.
+// Tensor maps of the token tensors for the tcgen05 kernel's copy engine (see kda_tma.cuh).  T == 0: nothing is ever copied,
+// the maps stay zeroed.
 // A prepared launch calls with the same pointers and strides every time, so the encoded maps are kept per thread
 // (a few entries, replaced round-robin) instead of going through the driver's encoder at every launch.
 struct MapKey {

@@ -34,12 +34,12 @@
 //
 // What bounds it: with 28 warps every warp issues about one instruction per ten cycles, so a chunk lasts as long as the chain
 // [kd ; qd] free -> operand tiles -> intra-chunk products -> inverse -> MMA2 over the two stages; the tensor pipe needs 970
-// cycles of it (the MMAs of a chunk depend on one another and still issue back to back).  Whole calls on a B200, first with
-// cumulative sums through shared memory and an inverse that waited for v, then with sums in the lanes of one warp and a third
-// q / k stage for raw gates, now with the decay in the 16-lane form, paired output stores, beta fetched ahead and the norms in
-// front of the gates: 8 x 1024 tokens at 64 heads, raw 415 / 392 / 347 us; 1 x 8192 at 96 heads, raw 770 / 696 / 604; 1 x 32768
-// at 16 heads with checkpoints, raw 990 / 949 / 857; 16 x U[128, 4096] at 32 heads, plain 547 / 512 / 489; 48 requests at 64
-// heads, plain 1792 / 1667 / 1616; 512 x 64 tokens at 64 heads, plain 2347 / 2302 / 2312 (start and end of a task).
+// cycles of it (the MMAs of a chunk depend on one another and still issue back to back).  Whole calls on a B200, with the
+// cumulative sums through shared memory and three barriers per chunk / as it is (two boxes): prepared launches of 8 x 1024 tokens at 64 heads,
+// raw 415 / 349 us, of 1 x 32768 at 16 heads with checkpoints, raw 985 / 865, of 48 requests at 64 heads, plain 2041 / 1919 (under the
+// power cap); one-shot calls of 1 x 8192 at 96 heads, raw 789 / 608, of 16 x U[128, 4096] at 32 heads, plain 625 / 568; a graph of
+// 512 x 64 tokens at 64 heads, plain 2345 / 2323 (start and end of a task).  The preparation warps react to where their code
+// lies: other text in a function that is never called there has moved long raw runs by 2.5 %.
 #include "kda_common.cuh"
 #include "kda_plan.cuh"
 #include "kda_tma.cuh"
@@ -168,8 +168,9 @@ __device__ __noinline__ void loader_drain(uint32_t bars, volatile int* abort_fla
 
 template <int FE>
 __device__ void role_loader(const ChunkParams& p, const TmaMaps& m, const Ctx& x, int lane) {
-  // Three independent copy streams (g; q and k; v), each with its own full / empty barrier pair per stage: the gate
-  // tile is free after step B of the chunk two back, q / k after step C, v only once MMA2 has read it.  ONE lane
+  // Three independent copy streams (g; q and k; v), each with its own full / empty barriers: the gate tile is free after
+  // step A of the chunk two back, q / k after step C of the chunk that had the stage (two back, three back with raw
+  // gates), v only once MMA2 has read it.  ONE lane
   // serves all three by polling the empty barriers without blocking: a blocking wait of one stream (or of a second
   // lane of this warp, which shares the warp's single scheduling slot) would delay the refill of the others by its
   // suspend time, and the refill latency of q / k sits on the chain  copy -> step B -> step C -> inverse -> MMA2.

@@ -36,15 +36,17 @@ constexpr int CUT_MAX_SEQS = 1024;       // sequences a cut plan is made for (be
 constexpr int N_CAND = 9;                // candidate piece lengths
 constexpr int MIN_PIECE_CHUNKS = 16;     // shorter pieces drown in the per-task cost
 constexpr int TASK_OVERHEAD = 3;         // start / end of a task, in chunk steps
-constexpr int DUAL_X8 = 9;               // a dual-chain chunk step without output rows costs 9 / 8 single-chain ones (measured 1.05-1.1)
+// A dual-chain chunk step without output rows in 1/8 single-chain ones.  An underestimate since the single-chain step became
+// shorter (slope from 128 to 256 chunks): raw gates 1.08 on 16 heads, 1.18 on 96; fp32 gates 1.28 and 1.26.
+constexpr int DUAL_X8 = 9;
 
 // chunk steps of the map of one piece of lp chunks: one dual-chain task, or two single-chain tasks
 __device__ __forceinline__ long long map_task_cost(int lp, int dual) {
   return dual ? (long long)(DUAL_X8 * lp + 7) / 8 + TASK_OVERHEAD : 2LL * (lp + TASK_OVERHEAD);
 }
 // One map of the scan chain, in 1/16 chunk steps.  An underestimate: a map takes 5.1 us value-first and 6.1 us key-first on
-// up to 16 heads (slope from 1 to 14 maps of one chain), about two chunk steps, so the model undercharges a cut by more
-// than one chunk step per map.
+// up to 16 heads (slope from 1 to 14 maps of one chain), about three chunk steps (1.7 us with fp32 gates, 2.0 with raw
+// ones), so the model undercharges a cut by two chunk steps per map.
 constexpr int SCAN_STEPS_X16 = 12;
 constexpr int LAUNCH_STEPS = 4;          // the scan launch and the second kernel launch, in chunk steps
 __host__ __device__ constexpr int cand_pieces(int k) { return k < 3 ? k + 2 : (k == 3 ? 6 : (k == 4 ? 8 : (k == 5 ? 12 : (k == 6 ? 16 : (k == 7 ? 24 : 32))))); }

@@ -86,8 +86,11 @@ def plan_bounds(T, H, first_rank, n_sms=148, max_pieces=8, task_overhead=3.0, fi
     return list(_plan(T, H, first_rank, n_sms, max_pieces, task_overhead, fixup_steps_per_chunk_head)[0])
 
 
-DUAL_COST = 1.40     # a dual-chain chunk step (with its two output tiles) in units of a single-chain one (measured inside the
-                     # 131072-token segment launches: 3.44 us against 2.47 us per chunk at 1.97 GHz)
+# A dual-chain chunk step (with its two output tiles) in units of a single-chain one.  Measured alone at 96 heads (slope from
+# 128 to 256 chunks): raw gates 3.21 us against 2.18 (1.47), fp32 gates 3.16 against 1.81 (1.75); the fix-up pass
+# 0.0033 and 0.0039 single-chain steps per chunk and head.  This charge and the fix-up's below are those of a longer
+# single-chain step.
+DUAL_COST = 1.40
 
 
 @functools.lru_cache(maxsize=256)        # the search costs milliseconds on the host; layouts repeat call after call

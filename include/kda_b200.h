@@ -56,9 +56,9 @@ enum {
   KDA_KERNEL_TCGEN05_TWO_TASK = 2  /* kda_segment_launch only (elsewhere the same as KDA_KERNEL_TCGEN05): chains L and
                               Tr of a mapped segment as two single-chain tasks.  With KDA_KERNEL_TCGEN05 a mapped
                               segment is ONE dual-chain task, both chains over one operand preparation
-                              (kda/b200/csrc/w3/base/cake_dual/kda_m128.cu:821-823): bit-identical results, about
-                              1.6 instead of 2 chunk steps per chunk; this value keeps the two-task scheme
-                              available as the cross-check */
+                              (kda/b200/csrc/w3/base/cake_dual/kda_m128.cu:821-823): bit-identical results, 1.4
+                              (raw gates) to 1.9 (fp32 gates) instead of 2 chunk steps per chunk; this value keeps
+                              the two-task scheme available as the cross-check */
 };
 
 /* Bits of status[0] (table validation, same meaning as kda/b200/kda_b200.py:56-62). */
