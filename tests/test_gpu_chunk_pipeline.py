@@ -123,7 +123,7 @@ def _rows_before(kda, token, value):
     return out[:, :token].float().cpu(), gold, kda.status_bits(launch)
 
 
-@pytest.mark.parametrize("value", [-1e9, float("-inf")])
+@pytest.mark.parametrize("value", [-90.0, -1400.0, -1500.0, -1e9, float("-inf")])
 @pytest.mark.parametrize("token", [16, 19, 22, 27, 31, 32 + 21, 64 + 25])
 def test_rows_in_front_of_a_reset_keep_their_decay(kda, token, value):
     """One token of a chunk's second half decays without bound (a state reset): the chunk is reported as out of range, and
