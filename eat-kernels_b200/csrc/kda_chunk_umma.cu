@@ -36,9 +36,9 @@
 // [kd ; qd] free -> operand tiles -> intra-chunk products -> inverse -> MMA2 over the two stages; the tensor pipe needs 970
 // cycles of it (the MMAs of a chunk depend on one another and still issue back to back).  Whole calls on a B200, with the
 // cumulative sums through shared memory and three barriers per chunk / as it is (two boxes): prepared launches of 8 x 1024 tokens at 64 heads,
-// raw 415 / 349 us, of 1 x 32768 at 16 heads with checkpoints, raw 985 / 865, of 48 requests at 64 heads, plain 2041 / 1919 (under the
-// power cap); one-shot calls of 1 x 8192 at 96 heads, raw 789 / 608, of 16 x U[128, 4096] at 32 heads, plain 625 / 568; a graph of
-// 512 x 64 tokens at 64 heads, plain 2345 / 2323 (start and end of a task).  The preparation warps react to where their code
+// raw 415 / 345 us, of 1 x 32768 at 16 heads with checkpoints, raw 985 / 883, of 48 requests at 64 heads, plain 2041 / 1920 (under the
+// power cap); one-shot calls of 1 x 8192 at 96 heads, raw 789 / 608, of 16 x U[128, 4096] at 32 heads, plain 625 / 571; a graph of
+// 512 x 64 tokens at 64 heads, plain 2345 / 2314 (start and end of a task).  The preparation warps react to where their code
 // lies: other text in a function that is never called there has moved long raw runs by 2.5 %.
 #include "kda_common.cuh"
 #include "kda_plan.cuh"
